@@ -37,8 +37,9 @@ typedef enum fs_status {
 } fs_status;
 
 /* Field solver kind.  DIRECT64 is the reference arithmetic in FP64 (bit-exact
- * with E_MQ_DirectSum); DIRECT32C is the FP32 pair kernel with compensation and
- * FP64 background; TREECODE64 / TREECODE32C are the barycentric Lagrange
+ * with E_MQ_DirectSum); DIRECT32C is held to 1e-6: FP64 cell expansions where
+ * 32 epsilon < L <= 5120 epsilon, else the FP32 pair kernel with compensation and
+ * FP64 background (the E a session hands out and batches always take the latter); TREECODE64 / TREECODE32C are the barycentric Lagrange
  * treecode of E_MQ_Treecode with an FP64 / FP32-compensated near field;
  * DIRECT64_OPEN is E_MQ_DirectSum_openbcs (src/FieldStructure.cpp:170-192),
  * open boundaries, bit-exact, field plugin only (L is ignored). */
@@ -179,7 +180,9 @@ typedef struct fs_sim fs_sim;
 fs_status fs_sim_create(const fs_sim_params* params, fs_sim** out);
 fs_status fs_sim_destroy(fs_sim* sim);
 /* nsteps x AMRSimulation::step (AMRSimulation_step.cpp:5-99), device resident,
- * synchronous on return. */
+ * synchronous on return.  FS_FIELD_DIRECT32C sessions evaluate the stage fields
+ * through cells and, after the call's last step, E once more by the FP32 pair
+ * kernel for fs_sim_export, which keeps E within rounding of the pairwise one. */
 fs_status fs_sim_step(fs_sim* sim, int nsteps);
 /* AMRSimulation::remesh (AMRSimulation_remesh.cpp:3-48) on the current state:
  * every species is interpolated onto its fresh mesh and the reduced-grid field

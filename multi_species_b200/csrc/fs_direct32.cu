@@ -44,6 +44,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "fs_bulk.cuh"
 #include "fs_device.cuh"
 
 namespace fsb {
@@ -64,55 +65,10 @@ constexpr int kNT = FS_NT;       // threads per CTA
 constexpr int kRMax = 8;         // largest number of targets per thread
 constexpr int kTBPad = kNT * kRMax;  // target counts are padded to a multiple of this
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// 1-D bulk copy global -> shared (TMA), completion signalled on `bar`.
-// Source and destination are 16-byte aligned and bytes is a multiple of 16.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, "
-        "p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Polls of one bounded mbarrier wait before it gives up (each poll may itself
-// suspend the thread for a short, hardware-chosen time).
-constexpr long long kMbarPolls = 1LL << 22;
 // The bound the pair kernels use for the waits on their source tiles.
 // fs_debug_set_wait_limits lowers it (0 = give up at once) so that tests can
 // drive the timeout path; the drain waits of that path always use kMbarPolls.
 __device__ long long g_mbar_polls = kMbarPolls;
-
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, long long polls) {
-    for (long long it = 0; it < polls; ++it)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-
 
 __device__ __forceinline__ double key_to_x(uint64_t k) { return __longlong_as_double((long long)k); }
 
@@ -817,6 +773,17 @@ class Direct32c final : public FieldEngine {
    public:
     Direct32c(double L, double eps) : L_(L), eps_(eps) {
         cbg_ = 1 / std::sqrt(L * L + 4 * eps * eps);
+        cells_ = cell_plan(L, eps, &plan_);
+        if (cells_) {
+            // the tables depend on L and eps alone; they are there before any
+            // (non-blocking) stream evaluates, captured or not
+            const size_t tab = (size_t)cell_table_offsets(plan_.Mc) * kCellTerms * kCellTerms;
+            tab_.ensure(tab + (size_t)kCellGroup * kCellTerms * kCellTerms);
+            buf_.tab = tab_.p;
+            buf_.child = tab_.p + tab;
+            cell_table(plan_, buf_.tab, buf_.child, nullptr);
+            FS_CUDA(cudaStreamSynchronize(nullptr));
+        }
         // tuning knob: targets per thread of the pair kernel (2, 4 or 8)
         if (const char* v = std::getenv("FS_B200_PAIR_TARGETS")) {
             const int r = std::atoi(v);
@@ -826,7 +793,15 @@ class Direct32c final : public FieldEngine {
 
 
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns, const Stage& stage,
-              cudaStream_t st) override {
+              cudaStream_t st, bool pairwise) override {
+        if (cells_ && !pairwise && nt > 0 && ns > 0) {
+            last_pairs = (double)nt * (double)ns;
+            last_nt_ = 0;
+            fin_ = Fin{};
+            reserve_cells(ns);
+            cell_field(plan_, buf_, d_t, nt, d_s, d_q, ns, stage, err_.p, st);
+            return;
+        }
         // a standalone launch: one persistent wave over about 32 items per CTA
         const int ntiles = (ns + kS - 1) / kS;
         const int nt_pad = (nt + kTBPad - 1) / kTBPad * kTBPad;
@@ -889,7 +864,13 @@ class Direct32c final : public FieldEngine {
             tperm = tiout_.p;
             FS_LAUNCHED(1);
         }
-        fin_ = Fin{true, nt, ns, nt_pad, ns > 0 ? nchunks : 1, tperm, stage};
+        fin_.pending = true;
+        fin_.nt = nt;
+        fin_.ns = ns;
+        fin_.nt_pad = nt_pad;
+        fin_.nchunks = ns > 0 ? nchunks : 1;
+        fin_.tperm = tperm;
+        fin_.stage = stage;
         if (ns <= 0) {
             FS_CUDA(cudaMemsetAsync(partial_.p, 0, sizeof(double) * nt_pad, st));
             return false;
@@ -905,17 +886,18 @@ class Direct32c final : public FieldEngine {
 
     void finalize(cudaStream_t st) override {
         if (!fin_.pending) return;
+        fin_.pending = false;
         const int T = 256;
         k_finalize32<<<(fin_.nt + T - 1) / T, T, 0, st>>>(partial_.p, fin_.nchunks, fin_.nt_pad, fin_.nt, info_.p,
                                                            pq_.p, qxsum_.p, fin_.ns, L_, cbg_, fin_.tperm, fin_.stage);
         FS_LAUNCHED(1);
-        fin_.pending = false;
     }
 
     int* error_flag() override { return err_.p; }
+    bool has_cells() const override { return cells_; }
 
-    // Pairs of the last evaluation (each evaluated); while profiling, also the
-    // band pairs among them, recorded as "pairs32_band_pairs".
+    // Pairs of the last evaluation; while profiling, after a pairwise one, also
+    // the band pairs among them, recorded as "pairs32_band_pairs".
     double actual_work(cudaStream_t st) override {
         if (last_pairs > 0 && last_nt_ > 0) prof_add_work("pairs32_band_pairs", band_pairs(st));
         return last_pairs;
@@ -948,7 +930,41 @@ class Direct32c final : public FieldEngine {
         return order_items(nitems, cost_.p, ids_.p, 2 * std::min(grid_, nitems), ordtmp_.p, tb, st);
     }
 
+    void reserve_common() {
+        if (err_.p) return;
+        err_.ensure(1);
+        FS_CUDA(cudaMemset(err_.p, 0, sizeof(int)));
+        counter_.ensure(1);
+        bandcount_.ensure(1);
+    }
+
+    void reserve_cells(int ns) {
+        reserve_common();
+        const int M = plan_.M, Mc = plan_.Mc;
+        ckeys_.ensure(2 * (size_t)ns);
+        iin_.ensure(ns);
+        iout_.ensure(ns);
+        part_.ensure(cell_partials(ns, M));
+        start_.ensure(M + 1);
+        coef_.ensure(2 * (size_t)(M + Mc) * kCellTerms);
+        const size_t sort = cell_sort_bytes(ns, M);
+        cub_.ensure(sort);
+        buf_.kin = ckeys_.p;
+        buf_.kout = ckeys_.p + ns;
+        buf_.iin = iin_.p;
+        buf_.iout = iout_.p;
+        buf_.part = part_.p;
+        buf_.start = start_.p;
+        buf_.mom = coef_.p;
+        buf_.loc = buf_.mom + (size_t)M * kCellTerms;
+        buf_.momc = buf_.loc + (size_t)M * kCellTerms;
+        buf_.locc = buf_.momc + (size_t)Mc * kCellTerms;
+        buf_.sort_tmp = cub_.p;
+        buf_.sort_bytes = sort;
+    }
+
     void reserve(int ns, int ns_pad, int nt_sep, int nt_pad, size_t npartial, int ntiles) {
+        reserve_common();
         kin_.ensure(ns);
         kout_.ensure(ns);
         iin_.ensure(ns);
@@ -963,12 +979,6 @@ class Direct32c final : public FieldEngine {
         tbase_.ensure(std::max(ntiles, 1));
         info_.ensure(nt_pad);
         partial_.ensure(npartial);
-        if (!err_.p) {
-            err_.ensure(1);
-            FS_CUDA(cudaMemset(err_.p, 0, sizeof(int)));
-            counter_.ensure(1);
-            bandcount_.ensure(1);
-        }
         const int nsort = std::max(ns, nt_sep);
         if (nt_sep) {
             tkin_.ensure(nt_sep);
@@ -1005,6 +1015,13 @@ class Direct32c final : public FieldEngine {
     DevBuf<TargetInfo> info_;
     DevBuf<int> err_, counter_;
     DevBuf<unsigned char> cub_;
+    // cell expansions
+    bool cells_ = false;
+    CellPlan plan_;
+    CellBuffers buf_;
+    DevBuf<uint32_t> ckeys_;
+    DevBuf<double> part_, coef_, tab_;
+    DevBuf<int> start_;
 };
 
 }  // namespace
@@ -1033,6 +1050,7 @@ FieldEngine* make_direct32c(double L, double eps) { return new Direct32c(L, eps)
 void set_mbar_polls(long long polls) {
     const long long v = polls < 0 ? kMbarPolls : polls;
     FS_CUDA(cudaMemcpyToSymbol(g_mbar_polls, &v, sizeof(v)));
+    set_cell_polls(polls);
 }
 
 constexpr int kNoAllocMaxPoints = 32768;
@@ -1071,7 +1089,30 @@ constexpr NoAllocLayout noalloc_layout() {
 }
 
 constexpr NoAllocLayout kNoAlloc = noalloc_layout();
-constexpr size_t kNoAllocBytes = kNoAlloc.total;
+
+// The same array laid out for an evaluation through cells (a call takes one
+// of the two forms), at the largest cell count.
+struct NoAllocCells {
+    size_t keys, idx, part, start, coef, tab, err, cub, total;
+};
+constexpr NoAllocCells noalloc_cells() {
+    NoAllocCells L{};
+    size_t o = 0;
+    const size_t n = kNoAllocMaxPoints, M = kCellMax, Mc = kCellMax / kCellGroup, p = kCellTerms;
+    L.keys = o;  o += align256(2 * n * sizeof(uint32_t));
+    L.idx = o;   o += align256(2 * n * sizeof(int));
+    L.part = o;  o += align256((n / 16 + M) * p * sizeof(double));
+    L.start = o; o += align256((M + 1) * sizeof(int));
+    L.coef = o;  o += align256(2 * (M + Mc) * p * sizeof(double));
+    L.tab = o;   o += align256((96 + Mc + kCellGroup) * p * p * sizeof(double));
+    L.err = o;   o += align256(sizeof(int));
+    L.cub = o;   o += kNoAllocCubBytes;
+    L.total = o;
+    return L;
+}
+constexpr NoAllocCells kNoAllocCells = noalloc_cells();
+static_assert(kCellMax / kCellGroup % 8 == 0, "table offsets: Mc needs no padding at the largest cell count");
+constexpr size_t kNoAllocBytes = kNoAlloc.total > kNoAllocCells.total ? kNoAlloc.total : kNoAllocCells.total;
 static_assert(kNoAllocMaxPoints % kTBPad == 0 && kNoAllocMaxPoints % kS == 0, "max size must fill whole blocks");
 
 // The scratch itself.  Host code must not use this symbol as an address: it
@@ -1115,6 +1156,40 @@ void direct32c_noalloc(double L, double eps, double* d_es, const double* d_x, co
     if (!d_es || !d_x || !d_q) fail(FS_ERR_ARG, "null device pointer");
     unsigned char* base = noalloc_scratch();
     auto at = [&](size_t off) { return base + off; };
+    auto finish = [&](int* err) {
+        int h = 0;
+        FS_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        FS_CUDA(cudaStreamSynchronize(st));
+        if (h) fail((fs_status)h, "device wait timed out in the field kernel");
+    };
+    Stage S;
+    S.kind = STAGE_STORE;
+    S.out = d_es;
+    CellPlan plan;
+    if (cell_plan(L, eps, &plan)) {
+        CellBuffers B;
+        B.kin = reinterpret_cast<uint32_t*>(at(kNoAllocCells.keys));
+        B.kout = B.kin + kNoAllocMaxPoints;
+        B.iin = reinterpret_cast<int*>(at(kNoAllocCells.idx));
+        B.iout = B.iin + kNoAllocMaxPoints;
+        B.part = reinterpret_cast<double*>(at(kNoAllocCells.part));
+        B.start = reinterpret_cast<int*>(at(kNoAllocCells.start));
+        B.mom = reinterpret_cast<double*>(at(kNoAllocCells.coef));
+        B.loc = B.mom + (size_t)plan.M * kCellTerms;
+        B.momc = B.loc + (size_t)plan.M * kCellTerms;
+        B.locc = B.momc + (size_t)plan.Mc * kCellTerms;
+        B.tab = reinterpret_cast<double*>(at(kNoAllocCells.tab));
+        B.child = B.tab + (size_t)cell_table_offsets(plan.Mc) * kCellTerms * kCellTerms;
+        B.sort_tmp = at(kNoAllocCells.cub);
+        B.sort_bytes = cell_sort_bytes(n, plan.M);
+        if (B.sort_bytes > kNoAllocCubBytes) fail(FS_ERR_UNSUPPORTED, "sort scratch larger than the static reserve");
+        int* cerr = reinterpret_cast<int*>(at(kNoAllocCells.err));
+        FS_CUDA(cudaMemsetAsync(cerr, 0, sizeof(int), st));
+        cell_table(plan, B.tab, B.child, st);
+        cell_field(plan, B, d_x, n, d_x, d_q, n, S, cerr, st);
+        finish(cerr);
+        return;
+    }
     uint64_t* kin = reinterpret_cast<uint64_t*>(at(kNoAlloc.kin));
     uint64_t* kout = reinterpret_cast<uint64_t*>(at(kNoAlloc.kout));
     int* iin = reinterpret_cast<int*>(at(kNoAlloc.iin));
@@ -1160,16 +1235,10 @@ void direct32c_noalloc(double L, double eps, double* d_es, const double* d_x, co
     const PairJob job{src, src64, tbase, info, partial, n, ntiles, tpc, nt_pad, L, (float)e2, (float)(e2 / 2),
                       (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, n};
     launch_pairs(R, dim3(tblocks, nchunks), st, job, err);
-    Stage S;
-    S.kind = STAGE_STORE;
-    S.out = d_es;
     const double cbg = 1 / std::sqrt(L * L + 4 * eps * eps);
     k_finalize32<<<(n + T - 1) / T, T, 0, st>>>(partial, nchunks, nt_pad, n, info, pq, qxsum, n, L, cbg, iout, S);
     FS_LAUNCHED(6);
-    int h = 0;
-    FS_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    FS_CUDA(cudaStreamSynchronize(st));
-    if (h) fail((fs_status)h, "device wait timed out in the field kernel");
+    finish(err);
 }
 
 }  // namespace fsb

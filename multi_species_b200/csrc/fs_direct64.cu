@@ -82,7 +82,7 @@ class Direct64Open final : public FieldEngine {
    public:
     explicit Direct64Open(double eps) : eps_(eps) {}
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns, const Stage& stage,
-              cudaStream_t st) override {
+              cudaStream_t st, bool) override {
         last_pairs = (double)nt * (double)ns;
         if (nt <= 0) return;
         const int blocks = (nt + kThreads64 - 1) / kThreads64;
@@ -102,7 +102,7 @@ class Direct64 final : public FieldEngine {
         norm_const_ = 1 / std::sqrt(L * L + 4 * eps * eps);
     }
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns,
-              const Stage& stage, cudaStream_t st) override {
+              const Stage& stage, cudaStream_t st, bool) override {
         last_pairs = (double)nt * (double)ns;
         if (nt <= 0) return;
         const int blocks = (nt + kThreads64 - 1) / kThreads64;

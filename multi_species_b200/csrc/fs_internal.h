@@ -205,14 +205,54 @@ struct PairJob {
     int nt;              // targets: the first nt of the nt_pad entries of info are real
 };
 
+// Cell expansions of the periodic direct sum (csrc/fs_cells.cu).
+constexpr int kCellTerms = 16;   // Chebyshev terms of a cell
+constexpr int kCellGroup = 16;   // cells of a group
+constexpr int kCellMax = 8192;   // cells at most
+struct CellPlan {
+    double L = 0, eps = 0, cbg = 0;
+    double h = 0, inv_h = 0, two_inv_h = 0;  // cell width, 1/h, 2/h
+    int M = 0, Mc = 0;                       // cells, groups
+};
+// Device scratch of one evaluation (raw views: the owner sizes them by the
+// functions below).
+struct CellBuffers {
+    uint32_t *kin = nullptr, *kout = nullptr;  // n
+    int *iin = nullptr, *iout = nullptr;       // n
+    double* part = nullptr;                    // cell_partials(n, M)
+    int* start = nullptr;                      // M + 1
+    double *mom = nullptr, *loc = nullptr;     // M * kCellTerms
+    double *momc = nullptr, *locc = nullptr;   // Mc * kCellTerms
+    double* tab = nullptr;                     // cell_table_offsets(Mc) * kCellTerms^2
+    double* child = nullptr;                   // kCellGroup * kCellTerms^2
+    void* sort_tmp = nullptr;
+    size_t sort_bytes = 0;                     // cell_sort_bytes(n, M)
+};
+// The cells of (L, eps); false where the pairwise kernel is used instead.
+bool cell_plan(double L, double eps, CellPlan* P);
+inline size_t cell_partials(int n, int M) { return ((size_t)(n + 15) / 16 + M) * kCellTerms; }
+__host__ __device__ inline int cell_table_offsets(int Mc) { return 96 + (Mc + 7) / 8 * 8; }
+size_t cell_sort_bytes(int n, int M);
+void cell_table(const CellPlan& P, double* tab, double* child, cudaStream_t st);
+// The whole evaluation: moments of the sources, the sums between cells, and E
+// at the targets through the stage epilogue.  *err is set by a bounded wait
+// that gave up.
+void cell_field(const CellPlan& P, const CellBuffers& B, const double* d_t, int nt, const double* d_s,
+                const double* d_q, int ns, const Stage& S, int* err, cudaStream_t st);
+void set_cell_polls(long long polls);
+
 class FieldEngine {
    public:
     virtual ~FieldEngine() = default;
     // Field at targets from sources (device pointers), result through the
     // stage epilogue, enqueued on `st`.  For targets == sources pass the same
     // pointer and nt == ns.
+    // `pairwise`: by the pairwise kernel where the engine has another form too.
     virtual void eval(const double* d_targets, int nt, const double* d_sources, const double* d_q,
-                      int ns, const Stage& stage, cudaStream_t st) = 0;
+                      int ns, const Stage& stage, cudaStream_t st, bool pairwise = false) = 0;
+    // Whether evaluations that are not `pairwise` go through cells (prepare()
+    // is always pairwise).
+    virtual bool has_cells() const { return false; }
     // Device int set non-zero by a kernel whose bounded wait gave up (or null).
     virtual int* error_flag() { return nullptr; }
     // Kernel-level evaluations of the last call (pairs for the direct sums;

@@ -1046,6 +1046,15 @@ struct Sim {
     double L = 0, t = 0, pairs = 0, evals = 0;
     std::vector<std::unique_ptr<SpeciesState>> sp;
     DevBuf<double> x, p, f, qw, e, xkA, xkB, pst, accX, accP, rx, rw, re;
+    // FP32c sessions take their stage fields through cells (csrc/fs_cells.cu)
+    // and keep the field of the next step's first stage in ek.  The field that
+    // leaves the session (e) is summed pairwise, once per call after its last
+    // step: on lattices of points the FP32 sums' rounding is coherent (1e-9 of E
+    // and more, where cells leave 1e-14), and e keeps following the pairwise
+    // session to 1e-10, as do positions and velocities, which integrate E.
+    // e_stale: the points have moved since e was formed.
+    DevBuf<double> ek;
+    bool via_cells = false, e_stale = false;
     DevBuf<int> status;
     std::unique_ptr<FieldEngine> field;
     cudaStream_t st = nullptr;
@@ -1183,7 +1192,9 @@ struct Sim {
         done.push_back(device);
     }
 
-    void create(const fs_sim_params& P, cudaStream_t external = nullptr) {
+    // `cells`: stage fields through cells where the field has them (a batch's
+    // members share pairwise launches instead).
+    void create(const fs_sim_params& P, cudaStream_t external, bool cells) {
         prm = P;
         if (P.num_species < 1 || P.num_species > 8) fail(FS_ERR_ARG, "num_species must be 1..8");
         if (!(P.xmax > P.xmin)) fail(FS_ERR_ARG, "xmax must exceed xmin");
@@ -1323,6 +1334,8 @@ struct Sim {
                 break;
             default: fail(FS_ERR_ARG, "unknown field kind");
         }
+        via_cells = cells && field->has_cells();
+        if (via_cells) ek.ensure(N);
         base.x = x.p;
         base.p = p.p;
         base.pst = pst.p;
@@ -1351,11 +1364,29 @@ struct Sim {
         int n;
         const double* q;
         Stage stage;
+        bool pairwise = false;
     };
 
     void run_call(const FieldCall& fc) {
-        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st);
+        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, fc.pairwise);
         account();
+    }
+
+    // The field of the points as they stand, pairwise, into e (see ek above).
+    void export_field() {
+        if (!e_stale) return;
+        Stage S = base;
+        S.kind = STAGE_STORE;
+        S.out = e.p;
+        const FieldCall fc = with_drive(FieldCall{x.p, N, qw.p, S, true}, t);
+        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, true);
+        if (profiling_enabled()) (void)field->actual_work(st);
+        e_stale = false;
+    }
+    // e was set from outside the steps: it is the next step's first field too.
+    void first_stage_field() {
+        e_stale = false;
+        if (via_cells) FS_CUDA(cudaMemcpyAsync(ek.p, e.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     }
 
     // Reduced grid (evaluate_field_uniform_grid): column sums, one field call
@@ -1382,13 +1413,14 @@ struct Sim {
         Stage S = base;
         S.kind = STAGE_STORE;
         S.out = re.p;
-        return with_drive(FieldCall{rx.p, U, rw.p, S}, t);
+        return with_drive(FieldCall{rx.p, U, rw.p, S, true}, t);
     }
     void reduced_post() {
         for (auto& s : sp) {
             k_scatter_reduced<<<blocks(s->n), kT, 0, st>>>(s->n, s->inv.p, re.p, e.p + s->start, status.p);
         }
         FS_LAUNCHED((long long)sp.size());
+        first_stage_field();
     }
     void reduced_field() {
         last_reduced_iter = iter;
@@ -1547,6 +1579,7 @@ struct Sim {
         upload(f, af);
         upload(qw, aq);
         for (auto* b : {&e, &xkA, &xkB, &pst, &accX, &accP}) b->ensure(N);
+        if (via_cells) ek.ensure(N);
         base.x = x.p;
         base.p = p.p;
         base.pst = pst.p;
@@ -1681,7 +1714,7 @@ struct Sim {
     void pre_call(int c) {
         if (c == 0) {
             Stage S1 = base;
-            k_rk_stage1<<<blocks(N), kT, 0, st>>>(N, S1, e.p, xkA.p);
+            k_rk_stage1<<<blocks(N), kT, 0, st>>>(N, S1, via_cells ? ek.p : e.p, xkA.p);
             FS_LAUNCHED(1);
         } else if (c == 3) {
             iter += 1;
@@ -1707,13 +1740,15 @@ struct Sim {
                 if (remeshing) return reduced_call();
                 Stage S = base;
                 S.kind = STAGE_STORE;
-                S.out = e.p;
+                S.out = via_cells ? ek.p : e.p;
                 return with_drive(FieldCall{x.p, N, qw.p, S}, t);
             }
         }
     }
     void post_call(int c) {
-        if (c == 3 && remeshing) reduced_post();
+        if (c != 3) return;
+        if (remeshing) reduced_post();
+        else e_stale = via_cells;
     }
 
     void step() {
@@ -1785,7 +1820,7 @@ fs_status fs_sim_create(const fs_sim_params* params, fs_sim** out) {
     if (!params || !out) return fsb::guard([] { fsb::fail(FS_ERR_ARG, "null argument"); });
     *out = nullptr;
     auto* s = new fs_sim();
-    fs_status rc = fsb::guard([&] { s->impl.create(*params); });
+    fs_status rc = fsb::guard([&] { s->impl.create(*params, nullptr, true); });
     if (rc != FS_OK) {
         delete s;
         return rc;
@@ -1812,6 +1847,7 @@ fs_status fs_sim_step(fs_sim* sim, int nsteps) {
         for (int k = 0; k < nsteps; ++k) {
             FS_CUDA(cudaEventRecord(S.ev0, S.st));
             S.step();
+            if (k == nsteps - 1) S.export_field();
             FS_CUDA(cudaEventRecord(S.ev1, S.st));
             S.check_status();
             float ms = 0.f;
@@ -1879,6 +1915,7 @@ fs_status fs_sim_export(fs_sim* sim, double* xs, double* ps, double* fs, double*
         if (!sim) fsb::fail(FS_ERR_ARG, "null sim");
         auto& S = sim->impl;
         FS_CUDA(cudaSetDevice(S.prm.device));
+        if (es) S.export_field();  // a step that failed midway through its call
         FS_CUDA(cudaStreamSynchronize(S.st));
         const size_t b = sizeof(double) * S.N;
         if (xs) FS_CUDA(cudaMemcpy(xs, S.x.p, b, cudaMemcpyDeviceToHost));
@@ -1898,7 +1935,11 @@ fs_status fs_sim_import_xp(fs_sim* sim, const double* xs, const double* ps, cons
         const size_t b = sizeof(double) * S.N;
         if (xs) fsb::h2d(S.x.p, xs, b);
         if (ps) fsb::h2d(S.p.p, ps, b);
-        if (es) fsb::h2d(S.e.p, es, b);
+        if (es) {
+            fsb::h2d(S.e.p, es, b);
+            S.first_stage_field();
+            FS_CUDA(cudaStreamSynchronize(S.st));
+        }
     });
 }
 
@@ -2057,7 +2098,7 @@ struct Batch {
         if (P.device != device) fail(FS_ERR_ARG, "simulation device differs from the batch device");
         FS_CUDA(cudaStreamSynchronize(st));
         auto s = std::make_unique<Sim>();
-        s->create(P, side[next_side++ % kSide]);
+        s->create(P, side[next_side++ % kSide], false);
         sims.push_back(std::move(s));
         ids.push_back(next_id);
         reset_graphs();
@@ -2712,7 +2753,7 @@ struct Pool {
             std::string err;
             try {
                 sim = std::make_unique<Sim>();
-                sim->create(r->prm);
+                sim->create(r->prm, nullptr, false);
             } catch (const FsError& e) {
                 err = e.msg.empty() ? "simulation set-up failed" : e.msg;
             } catch (const std::exception& e) {

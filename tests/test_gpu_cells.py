@@ -1,0 +1,83 @@
+"""The FP32-compensated direct sum through cell expansions (L between 32 and
+5120 epsilon) against the oracle's FP64 pairwise sum, and the sessions whose
+stage fields go through it."""
+import numpy as np
+import pytest
+
+import oracle as O
+import multi_species_b200 as M
+from multi_species_b200 import decks
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(kind, n, L, rng):
+    if kind == "cell":      # all in one cell, away from its middle
+        return rng.uniform(0.2, 0.21, n) * 0.6 * L / 5120
+    if kind == "cluster":   # half in a few cells, the rest over several periods
+        return np.concatenate([rng.normal(L / 3, 0.003 * L, n // 2), rng.uniform(-2 * L, 3 * L, n - n // 2)])
+    if kind == "lattice":   # coincident points, half-period partners, cell edges
+        return (rng.integers(0, 64, n) / 64 + rng.integers(-2, 3, n)) * L
+    return rng.uniform(-L, 2 * L, n)
+
+
+@pytest.mark.parametrize("ratio,n,nt,kind", [
+    (32.5, 3000, 0, "uniform"), (63.0, 257, 33, "lattice"), (251.3, 1, 0, "uniform"), (251.3, 2, 7, "uniform"),
+    (251.3, 15, 0, "lattice"), (251.3, 16, 1, "cell"), (251.3, 255, 0, "cell"), (251.3, 256, 300, "cluster"),
+    (251.3, 4097, 0, "cluster"), (1570.8, 17, 0, "uniform"), (1570.8, 20000, 513, "uniform"),
+    (1570.8, 4097, 0, "lattice"), (5119.0, 5000, 0, "cluster"),
+    # just outside on either side: the pairwise kernel
+    (32.0, 1000, 0, "uniform"), (5121.0, 1000, 0, "uniform")])
+def test_cells_match_the_fp64_sum(ratio, n, nt, kind):
+    """16 Chebyshev terms on cells of epsilon / 1.6 leave (6.5)^-16 = 1e-13 of a
+    pair's charge; below L = 64 epsilon the cell pair across the half period adds
+    up to 0.06 (epsilon / L)^2 / 256^3 = 4e-12 of the charge.  The pairwise kernel
+    is held to its own 1e-9 of the band charge."""
+    rng = np.random.default_rng(n + int(ratio))
+    L = 4 * np.pi
+    eps = L / ratio
+    s = _points(kind, n, L, rng)
+    q = rng.normal(size=n) / n
+    t = _points(kind, nt, L, rng) if nt else s
+    e = M.E_MQ_DirectSum_B200(L, eps, "fp32c").evaluate(t, s, q)
+    ref = O.direct_sum(L, eps, t, s, q)
+    tol = 2e-9 if not 32 < ratio <= 5120 else (1e-11 if ratio < 64 else 1e-12)
+    assert np.max(np.abs(e - ref)) <= tol * np.sum(np.abs(q))
+
+
+def test_nan_charge_reaches_every_target():
+    L = 4 * np.pi
+    x = np.linspace(0, L, 100, endpoint=False)
+    q = np.full(100, 0.1)
+    q[17] = np.nan
+    assert np.all(np.isnan(M.E_MQ_DirectSum_B200(L, 0.05, "fp32c").evaluate(x + 0.01, x, q)))
+
+
+def test_session_is_the_same_however_its_steps_are_called():
+    """Stage fields through cells, E handed out summed pairwise after a call's
+    last step: four steps in one call and one by one agree bit for bit, with
+    and without a remesh among them."""
+    for period in (3, 100):
+        d = decks.two_stream(h=4, ph=1, remesh_period=period)
+        a, b = M.Simulation(d, "direct32c"), M.Simulation(d, "direct32c")
+        a.step(4)
+        for _ in range(4):
+            b.step(1)
+            b.state()
+        sa, sb = a.state(), b.state()
+        for k in ("xs", "ps", "fs", "q_ws", "es"):
+            assert np.array_equal(sa[k], sb[k]), (period, k)
+
+
+def test_imported_field_is_the_next_steps_first():
+    d = decks.two_stream(h=4, ph=1, remesh_period=100)
+    a, b = M.Simulation(d, "direct32c"), M.Simulation(d, "direct64")
+    es = np.sin(0.2 * a.state()["xs"])
+    for s in (a, b):
+        s.step(2)
+        s.import_xp(es=es)
+        assert np.array_equal(s.state()["es"], es)
+        s.step(1)
+    sa, sb = a.state(), b.state()
+    for k in ("xs", "ps"):
+        assert np.linalg.norm(sa[k] - sb[k]) <= 1e-8 * np.linalg.norm(sb[k]), k
