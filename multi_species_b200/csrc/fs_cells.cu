@@ -34,7 +34,7 @@
 #include <cmath>
 
 #include "fs_bulk.cuh"
-#include "fs_device.cuh"
+#include "fs_cells.cuh"
 
 namespace fsb {
 
@@ -52,15 +52,6 @@ static_assert(kP == 16 && kC == 16, "thread maps below");
 
 // Bound of the waits on the moment copies (fs_debug_set_wait_limits).
 __device__ long long g_cell_polls = kMbarPolls;
-
-// Position in [0, L] (NaN stays NaN), its cell and its place in the cell.
-__device__ __forceinline__ double cell_wrap(double x, double L) {
-    const double w = x - L * floor(x / L);
-    return w < 0.0 ? 0.0 : (w > L ? L : w);
-}
-__device__ __forceinline__ int cell_of(double w, const CellPlan& P) {
-    return min(max((int)(w * P.inv_h), 0), P.M - 1);
-}
 
 __global__ void k_cell_keys(CellPlan P, const double* __restrict__ x, int n, uint32_t* __restrict__ key,
                             int* __restrict__ idx) {
@@ -310,24 +301,6 @@ __global__ void __launch_bounds__(kPairT) k_cell_pairs(CellSums J, int* __restri
     else cell_near(J, b - nf, S, err);
 }
 
-// sum_l a[l] T_l(x) by Clenshaw's recurrence; a is 16-byte aligned.
-__device__ __forceinline__ double cheb_sum(const double* __restrict__ a, double x) {
-    const double2* a2 = reinterpret_cast<const double2*>(a);
-    double b1 = 0.0, b2 = 0.0;
-    const double x2 = x + x;
-#pragma unroll
-    for (int h = kP / 2 - 1; h > 0; --h) {
-        const double2 c = __ldg(a2 + h);
-        const double u = fma(x2, b1, c.y - b2);
-        b2 = fma(x2, u, c.x - b1);
-        b1 = b2;
-        b2 = u;
-    }
-    const double2 c = __ldg(a2);
-    const double u = fma(x2, b1, c.y - b2);
-    return fma(x, u, c.x - b1);
-}
-
 // E at the targets (in the caller's order: coalesced stage arrays; a cell's
 // coefficients are one 128-byte line) through the stage epilogue.
 __global__ void __launch_bounds__(256) k_cell_eval(CellPlan P, const double* __restrict__ x, int n,
@@ -343,20 +316,37 @@ __global__ void __launch_bounds__(256) k_cell_eval(CellPlan P, const double* __r
     apply_stage(S, i, E);
 }
 
-// One CTA per offset: G on the 16 x 16 Chebyshev nodes of the two cells, then
-// both sides to coefficients.  The last kC CTAs form the child matrices.
+// G on the 16 x 16 Chebyshev nodes of two cells of width hh whose centres are d0
+// apart, both sides to coefficients, as T[k][l] (a CTA of kPP threads).
+__device__ void offset_table(const CellPlan& P, double d0, double hh, bool zero, double* __restrict__ out) {
+    __shared__ double A[kP][kP + 1], C[kP][kP + 1], X[kP][kP + 1];
+    const int t = threadIdx.x, a = t >> 4, b = t & 15;
+    C[a][b] = cospi((a + 0.5) * b / kP) * (b ? 2.0 : 1.0) / kP;  // node a's share of coefficient b
+    const double na = cospi((a + 0.5) / kP), nb = cospi((b + 0.5) / kP);
+    double d = d0 + (na - nb) * (0.5 * hh);
+    d -= P.L * rint(d / P.L);
+    A[a][b] = zero ? 0.0 : d / (2.0 * sqrt(d * d + P.eps * P.eps)) - P.cbg * d;
+    __syncthreads();
+    double s = 0.0;  // X[l][b] = sum_a C[a][l] A[a][b], thread (l = a, b)
+    for (int n = 0; n < kP; ++n) s = fma(C[n][a], A[n][b], s);
+    X[a][b] = s;
+    __syncthreads();
+    s = 0.0;  // T[k][l], thread (k = a, l = b)
+    for (int n = 0; n < kP; ++n) s = fma(C[n][a], X[b][n], s);
+    out[t] = s;
+}
+
+// One CTA per offset of the two levels; the last kC CTAs form the child matrices.
 __global__ void __launch_bounds__(kPP) k_cell_table(CellPlan P, double* __restrict__ tab,
                                                     double* __restrict__ child) {
-    __shared__ double A[kP][kP + 1], C[kP][kP + 1], X[kP][kP + 1];  // C[a][k]: node a's share of coefficient k
-    const int t = threadIdx.x, a = t >> 4, b = t & 15;
-    C[a][b] = cospi((a + 0.5) * b / kP) * (b ? 2.0 : 1.0) / kP;
     const int o = blockIdx.x;
     const int noff = cell_table_offsets(P.Mc);
-    const double na = cospi((a + 0.5) / kP), nb = cospi((b + 0.5) / kP);
     if (o >= noff) {
-        // T_k of child node a in the group, k = b: then its Chebyshev coefficients
+        __shared__ double A[kP][kP + 1];
+        const int t = threadIdx.x, a = t >> 4, b = t & 15;
+        // T_k of child node a's place in the group, k = b: then its coefficients
         const int c = o - noff;
-        const double y = (na + (double)(2 * c + 1 - kC)) * (1.0 / kC);
+        const double y = (cospi((a + 0.5) / kP) + (double)(2 * c + 1 - kC)) * (1.0 / kC);
         double u = 1.0, v = y;
         for (int k = 0; k < b; ++k) {
             const double z = fma(2.0 * y, v, -u);
@@ -366,12 +356,13 @@ __global__ void __launch_bounds__(kPP) k_cell_table(CellPlan P, double* __restri
         A[a][b] = u;
         __syncthreads();
         double s = 0.0;  // thread (k = a, l = b)
-        for (int n = 0; n < kP; ++n) s = fma(C[n][b], A[n][a], s);
+        for (int n = 0; n < kP; ++n)
+            s = fma(cospi((n + 0.5) * b / kP) * (b ? 2.0 : 1.0) / kP, A[n][a], s);
         child[((size_t)c * kP + a) * kP + b] = s;
         return;
     }
-    double d0 = 0.0, hh = P.h;  // distance of the cells' centres, cell width
-    bool zero = false;
+    double d0, hh = P.h;
+    bool zero;
     if (o < kNearOff) {
         d0 = (o - 32) * P.h;
         zero = o == 0;
@@ -384,17 +375,12 @@ __global__ void __launch_bounds__(kPP) k_cell_table(CellPlan P, double* __restri
         d0 = m * hh;
         zero = m <= 1 || m >= P.Mc - 1 || m == P.Mc / 2;
     }
-    double d = d0 + (na - nb) * (0.5 * hh);
-    d -= P.L * rint(d / P.L);
-    A[a][b] = zero ? 0.0 : d / (2.0 * sqrt(d * d + P.eps * P.eps)) - P.cbg * d;
-    __syncthreads();
-    double s = 0.0;  // X[l][b] = sum_a C[a][l] A[a][b], thread (l = a, b)
-    for (int n = 0; n < kP; ++n) s = fma(C[n][a], A[n][b], s);
-    X[a][b] = s;
-    __syncthreads();
-    s = 0.0;  // T[k][l], thread (k = a, l = b)
-    for (int n = 0; n < kP; ++n) s = fma(C[n][a], X[b][n], s);
-    tab[(size_t)o * kPP + t] = s;
+    offset_table(P, d0, hh, zero, tab + (size_t)o * kPP);
+}
+
+// One CTA per cell offset 0 .. M - 1.
+__global__ void __launch_bounds__(kPP) k_offset_table(CellPlan P, double* __restrict__ tab) {
+    offset_table(P, blockIdx.x * P.h, P.h, false, tab + (size_t)blockIdx.x * kPP);
 }
 
 int key_bits(int M) {
@@ -432,6 +418,11 @@ size_t cell_sort_bytes(int n, int M) {
 
 void cell_table(const CellPlan& P, double* tab, double* child, cudaStream_t st) {
     k_cell_table<<<cell_table_offsets(P.Mc) + kC, kPP, 0, st>>>(P, tab, child);
+    FS_LAUNCHED(1);
+}
+
+void cell_offset_table(const CellPlan& P, double* tab, cudaStream_t st) {
+    k_offset_table<<<P.M, kPP, 0, st>>>(P, tab);
     FS_LAUNCHED(1);
 }
 

@@ -234,6 +234,8 @@ inline size_t cell_partials(int n, int M) { return ((size_t)(n + 15) / 16 + M) *
 __host__ __device__ inline int cell_table_offsets(int Mc) { return 96 + (Mc + 7) / 8 * 8; }
 size_t cell_sort_bytes(int n, int M);
 void cell_table(const CellPlan& P, double* tab, double* child, cudaStream_t st);
+// T^{(m)}[k][l] for every cell offset m = 0 .. M - 1 (M * kCellTerms^2).
+void cell_offset_table(const CellPlan& P, double* tab, cudaStream_t st);
 // The whole evaluation: moments of the sources, the sums between cells, and E
 // at the targets through the stage epilogue.  *err is set by a bounded wait
 // that gave up.

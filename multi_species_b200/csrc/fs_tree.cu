@@ -34,24 +34,13 @@
 #include <cmath>
 #include <vector>
 
-#include "fs_device.cuh"
+#include "fs_tree.cuh"
 
 namespace fsb {
 
 namespace {
 
-constexpr int kMaxDegree = 16;
-constexpr int kMaxDepth = 60;
-constexpr int kFarCap = 256;   // far-list entries per leaf
-constexpr int kNearCap = 64;   // near-list entries per leaf
 constexpr int kChunk = 8192;   // member points per moment work item
-
-struct TNode {
-    double x0, x1, xc;
-    int m0, m1;       // inclusive member range in sorted order
-    int child0, child1;
-    int parent, level;
-};
 
 // Per-instance constants (device array of 2 x (kMaxDegree+1) doubles):
 //   cheb[k] = cos(k pi / P) from the host C library, w[k] = (-1)^k (1/2 at the ends).
@@ -941,6 +930,7 @@ class Treecode final : public FieldEngine {
         FS_CUDA(cudaStreamSynchronize(nullptr));  // the copy lands before the engine's non-blocking streams read it
         norm_ = std::sqrt(L * L + 4 * eps * eps) / L;
         cbg_ = 1 / std::sqrt(L * L + 4 * eps * eps);
+        cells_.init(L, eps);
     }
 
     int* error_flag() override { return err_.p; }
@@ -988,7 +978,13 @@ class Treecode final : public FieldEngine {
         k_moment_reduce<<<(cap_nodes + T - 1) / T, T, 0, st>>>(nodes_.p, meta_.p, cap_nodes, item_start_.p, P_,
                                                               mpart_.p, mom_.p);
         k_copy_meta_error<<<1, 1, 0, st>>>(meta_.p, err_.p);
-        if (!fp32_) {
+        if (through_cells(n)) {
+            const TreeView T{nodes_.p, leaves_.p, meta_.p, leaf_of_.p, far_.p, far_n_.p, near_.p, near_n_.p,
+                             mom_.p, consts_.p, sx_.p, lam_.p, iout_.p, n, P_, cap_leaves};
+            ProfScope prof(fp32_ ? "k_near32" : "k_far_near64", st, last_pairs);
+            cells_.eval(T, N0_, norm_, stage, st);
+            FS_LAUNCHED(9);
+        } else if (!fp32_) {
             ProfScope prof("k_far_near64", st, last_pairs);
             k_far_near64<<<(n + 127) / 128, 128, 0, st>>>(nodes_.p, meta_.p, leaf_of_.p, leaves_.p, far_.p, far_n_.p,
                                                          near_.p, near_n_.p, mom_.p, consts_.p, sx_.p, lam_.p,
@@ -1035,6 +1031,15 @@ class Treecode final : public FieldEngine {
     }
 
    private:
+    // Sums through cells (csrc/fs_treecells.cu) where leaves hold many points
+    // per cell.  The FP32c form changes over where its FP32 near sums are
+    // themselves within 6e-10 of the FP64 treecode (1.7e-9 at 32 points per
+    // epsilon, 5e-10 at 126, 4e-11 at 2000), so that E does not step there.
+    bool through_cells(int n) const {
+        if (!cells_.ready()) return false;
+        const double per_eps = n * eps_ / L_;  // points per epsilon at uniform density
+        return fp32_ ? per_eps >= 128 : per_eps >= 16;
+    }
 
     void reserve(int n, int cap_nodes, int cap_leaves, int cap_items) {
         kin_.ensure(n);
@@ -1097,6 +1102,7 @@ class Treecode final : public FieldEngine {
     int near_grid_ = 0;
     int cap_leaves_ = 0;
     DevBuf<TNode> nodes_;
+    TreeCells cells_;
     DevBuf<unsigned char> cub_;
 };
 
