@@ -519,21 +519,27 @@ __global__ void k_far32(const TNode* __restrict__ nodes, const int* __restrict__
     efar[j] = norm * far;
 }
 
-// FP32-compensated form, near part: one CTA per (leaf, block of
-// kNearThreads x kNearR targets), kNearR targets per thread.
+// FP32-compensated form, near part: a CTA per (leaf, block of kNearThreads x
+// kNearR targets), or two with two targets per thread each, the near list
+// shared by several, where the targets are few.
 //   K_tc(d) / norm = d/(2 sqrt(d^2+eps^2)) - c d,  d = xt - x_j  (xt = image of x_i)
 // The linear term c d is summed exactly in FP64 from prefix sums of lambda and
-// lambda x.  For each near leaf, when every target of the CTA sees the whole
-// leaf in one periodic image and within the band |d| <= band (the usual case:
-// near leaves are neighbours a few leaf widths away), the pairs are
-// lambda/2 d y, y = rsqrt(d^2+eps^2), accumulated in packed FP32x2 over two
-// targets with Kahan compensation per tile and reduced in FP64 across tiles.
-// Otherwise every target of the CTA takes the general path for that leaf: the
-// leaf's sources are cut where their image changes (at most three images), and
-// beyond the band the sign part sign(d) lambda/2 is summed exactly in FP64 while
-// the kernel accumulates -+ lambda/2 c(v) (c = v/2 + v^2/8, v = eps^2 y^2).
-// Sources are staged through shared memory as FP32 offsets from an FP64 tile
-// base; each image's target offset is formed in FP64 before rounding.
+// lambda x.  For each near leaf, when every target of the block sees the whole
+// leaf in one periodic image and within the band |d| <= band (leaves narrower
+// than the band), the pairs are lambda/2 d y, y = rsqrt(d^2+eps^2), accumulated
+// in packed FP32x2 over two targets with Kahan compensation per tile and reduced
+// in FP64 across tiles.  Otherwise the block takes the general path for that
+// leaf: the leaf's sources are cut where their image changes (at most three
+// images), and beyond the band the sign part sign(d) lambda/2 is summed exactly
+// in FP64 while the kernel accumulates -+ lambda/2 c(v) (c = v/2 + v^2/8, v =
+// eps^2 y^2).  Sources are staged through shared memory as FP32 offsets from an
+// FP64 tile base; each image's target offset is formed in FP64 before rounding.
+//
+// What bounds it: one MUFU.RSQ per pair (16/clk/SM), and for wide leaves the
+// latency of the Kahan chain, which wants warps: 99,000 points (leaves of 50
+// epsilon) 2.27 ms with four targets per thread walked one by one, 0.99 ms in
+// packed pairs, 0.45 ms with the near lists shared by eight CTAs, the results
+// equal (the shared lists' FP64 additions to 1e-16).
 #ifndef FS_NEAR_THREADS
 #define FS_NEAR_THREADS 128
 #endif
@@ -543,20 +549,19 @@ __global__ void k_far32(const TNode* __restrict__ nodes, const int* __restrict__
 constexpr int kNearThreads = FS_NEAR_THREADS;
 constexpr int kNearR = FS_NEAR_R;
 constexpr int kNearBlock = kNearThreads * kNearR;
+static_assert(kNearR == 4, "two pairs of targets per thread");
 constexpr int kNearTile = 256;
 constexpr double kNearBand = 24.0;
-// near items taken by a persistent grid in decreasing order of work (1) or one
-// CTA per item in leaf order (0).  At 6.3M points (1) measured 0.5% slower per
-// treecode step than (0): the plain grid of ~12k CTAs leaves little tail.
-#ifndef FS_NEAR_ORDER
-#define FS_NEAR_ORDER 0
-#endif
-constexpr bool kNearOrder = FS_NEAR_ORDER;
-
-struct NearImage {
-    double xt;    // target coordinate in this image
-    int start;    // first source index of the image's subrange
-    int U1, U2;   // band [U1, U2): |d| <= band
+constexpr int kNearSplit = 16;  // below this many target blocks per SM a thread takes two targets
+// CTAs per SM that sharing near lists aims at, and parts of a list at most (12:
+// 12 to 29% slower at 100,000 to 400,000 points; 16 parts no faster)
+constexpr int kNearCtas = 24, kNearParts = 8;
+// The images of a near leaf's sources as one target sees them, at most three:
+// image k holds sources [start[k], start[k + 1]) at target coordinate xt[k],
+// with the band |d| <= band at [U1[k], U2[k]).
+struct NearImages {
+    double xt[3];
+    int start[4], U1[3], U2[3];
 };
 
 __device__ __forceinline__ int lower_bound_d(const double* __restrict__ a, int lo, int hi, double v) {
@@ -581,81 +586,173 @@ __device__ __forceinline__ double range_sum(const double* __restrict__ incl, int
     return incl[e - 1] - (a > 0 ? incl[a - 1] : 0.0);
 }
 
-// General path for one target and one near leaf (all threads of the CTA call
-// it together: it stages tiles through `sh` with barriers).
-__device__ void near_general(const TNode& nd, double x, const double* __restrict__ sx,
-                             const double* __restrict__ lam, const double* __restrict__ pl,
-                             const double* __restrict__ plx, double L, double band, double cbg, float eps2, float a1,
-                             float a2, float4* sh, double& exact, double& fp, int* __restrict__ err) {
-    NearImage im[3];
-    int nim = 0;
-    int a = nd.m0;
-    while (a <= nd.m1 && nim < 3) {
-        // image of source j: m_j = round((x - x_j) / L), the reference's
-        // choice (z - round(z)); m_j is non-increasing in j
-        const double m = round((x - sx[a]) / L);
-        const double xt = x - m * L;
-        int e;  // first source of the next image
-        {
-            int lo = a + 1, hi = nd.m1 + 1;
-            while (lo < hi) {
-                const int mid = lo + ((hi - lo) >> 1);
-                if (round((x - sx[mid]) / L) < m) hi = mid;
-                else lo = mid + 1;
+// Cuts the leaf's sources where their image changes, finds each image's band
+// and adds the exact terms: the linear term and, beyond the band, the sign part.
+__device__ __forceinline__ void near_images(const TNode& nd, double x, const double* __restrict__ sx,
+                                            const double* __restrict__ pl, const double* __restrict__ plx, double L,
+                                            double band, double cbg, NearImages& im, double& exact,
+                                            int* __restrict__ err) {
+    int a = nd.m0, nim = 0;
+    const double xlast = sx[nd.m1];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        im.start[k] = INT_MAX;
+        im.U1[k] = im.U2[k] = 0;
+        im.xt[k] = k ? im.xt[k - 1] : 0.0;
+        if (a <= nd.m1) {
+            // image of source j: m_j = round((x - x_j) / L), the reference's
+            // choice (z - round(z)); m_j is non-increasing in j
+            const double m = round((x - sx[a]) / L);
+            const double xt = x - m * L;
+            int e = nd.m1 + 1;  // first source of the next image
+            if (round((x - xlast) / L) < m) {
+                int lo = a + 1, hi = nd.m1 + 1;
+                while (lo < hi) {
+                    const int mid = lo + ((hi - lo) >> 1);
+                    if (round((x - sx[mid]) / L) < m) hi = mid;
+                    else lo = mid + 1;
+                }
+                e = lo;
             }
-            e = lo;
+            // most leaves lie wholly inside the band or wholly to one side
+            const double first = sx[a], last = sx[e - 1];
+            const int U1 = first >= xt - band ? a : (last < xt - band ? e : lower_bound_d(sx, a, e, xt - band));
+            const int U2 = last <= xt + band ? e : (U1 < e && sx[U1] <= xt + band ? upper_bound_d(sx, U1, e, xt + band)
+                                                                                   : U1);  // first x_j > xt + band
+            exact += 0.5 * (range_sum(pl, a, U1) - range_sum(pl, U2, e)) -
+                     cbg * (xt * range_sum(pl, a, e) - range_sum(plx, a, e));
+            im.xt[k] = xt;
+            im.start[k] = a;
+            im.U1[k] = U1;
+            im.U2[k] = U2;
+            ++nim;
+            a = e;
         }
-        const int U1 = lower_bound_d(sx, a, e, xt - band);
-        const int U2 = upper_bound_d(sx, U1, e, xt + band);  // first x_j > xt + band
-        exact += 0.5 * (range_sum(pl, a, U1) - range_sum(pl, U2, e)) -
-                 cbg * (xt * range_sum(pl, a, e) - range_sum(plx, a, e));
-        im[nim].xt = xt;
-        im[nim].start = a;
-        im[nim].U1 = U1;
-        im[nim].U2 = U2;
-        ++nim;
-        a = e;
     }
+    im.start[3] = INT_MAX;
     if (a <= nd.m1) atomicCAS(err, 0, (int)FS_ERR_TREE);
-    for (int k = nim; k < 3; ++k) {
-        im[k].xt = im[nim - 1].xt;
-        im[k].start = INT_MAX;
-        im[k].U1 = im[k].U2 = 0;
+}
+
+// Sources [t0, t0 + cnt) as one target sees them: its offset when they share an
+// image, and 1 (beyond the band on the left), 2 (right), 3 (in the band) when
+// they also share a side; 0 otherwise.
+__device__ __forceinline__ int near_side(const NearImages& im, int t0, int cnt, double base, float& tau) {
+    int side = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (t0 >= im.start[k] && (im.start[k + 1] == INT_MAX || t0 + cnt <= im.start[k + 1])) {
+            tau = (float)(im.xt[k] - base);
+            side = t0 + cnt <= im.U1[k] ? 1 : (t0 >= im.U2[k] ? 2 : (t0 >= im.U1[k] && t0 + cnt <= im.U2[k] ? 3 : 0));
+        }
     }
-    for (int t0 = nd.m0; t0 <= nd.m1; t0 += kNearTile) {
+    return side;
+}
+
+// One tile for one target, image and side per source.
+__device__ void near_mixed(const NearImages& im, int t0, int cnt, double base, const float4* sh, float eps2,
+                           float& acc, float& ncmp) {
+    const float tau0 = (float)(im.xt[0] - base), tau1 = (float)(im.xt[1] - base), tau2 = (float)(im.xt[2] - base);
+    for (int k = 0; k < cnt; ++k) {
+        const int jj = t0 + k;
+        const bool g1 = jj >= im.start[1], g2 = jj >= im.start[2];
+        const float tr = g2 ? tau2 : (g1 ? tau1 : tau0);
+        const int U1 = g2 ? im.U1[2] : (g1 ? im.U1[1] : im.U1[0]);
+        const int U2 = g2 ? im.U2[2] : (g1 ? im.U2[1] : im.U2[0]);
+        const float4 e = sh[k];
+        const float d = tr - e.x;
+        const float y = rsqrt_approx(fmaf(d, d, eps2));
+        const float z = __fmul_rn(y, y);
+        const float c = __fmul_rn(z, fmaf(z, e.w, e.z));
+        const float v = (jj < U1) ? -c : ((jj >= U2) ? c : __fmul_rn(e.y, __fmul_rn(d, y)));
+        const float w = __fadd_rn(v, ncmp);
+        const float t = __fadd_rn(acc, w);
+        ncmp = __fsub_rn(w, __fsub_rn(t, acc));
+        acc = t;
+    }
+}
+
+// General path for a pair of targets and one near leaf (all threads of the CTA
+// call it together: it stages tiles through `sh` with barriers).  Most tiles are
+// of one side for all of a warp's targets, and these run in packed FP32x2; the
+// others go pair by pair.  The Kahan compensation is kept negated.
+__device__ void near_general2(const TNode& nd, const double (&x)[2], const double* __restrict__ sx,
+                              const double* __restrict__ lam, const double* __restrict__ pl,
+                              const double* __restrict__ plx, double L, double band, double cbg, float eps2, float a1,
+                              float a2, float4 (*sh)[kNearTile], double* exact, double* fp, int* __restrict__ err) {
+    NearImages im[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) near_images(nd, x[h], sx, pl, plx, L, band, cbg, im[h], exact[h], err);
+    constexpr int kPer = kNearTile / kNearThreads;
+    double nx[kPer], nl[kPer];
+    double nbase = 0.0;
+    auto fetch = [&](int t0) {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int j = t0 + threadIdx.x + i * kNearThreads;
+            nx[i] = (j <= nd.m1) ? sx[j] : 0.0;
+            nl[i] = (j <= nd.m1) ? lam[j] : 0.0;
+        }
+        nbase = sx[t0];
+    };
+    fetch(nd.m0);
+    int buf = 0;
+    for (int t0 = nd.m0; t0 <= nd.m1; t0 += kNearTile, buf ^= 1) {
         const int cnt = min(kNearTile, nd.m1 - t0 + 1);
-        const double base = sx[t0];
-        __syncthreads();
-        for (int k = threadIdx.x; k < cnt; k += kNearThreads) {
-            const float lh = (float)(0.5 * lam[t0 + k]);
-            sh[k] = make_float4((float)(sx[t0 + k] - base), lh, lh * a1, lh * a2);
+        const double base = nbase;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const float lh = (float)(0.5 * nl[i]);
+            sh[buf][threadIdx.x + i * kNearThreads] =
+                make_float4((float)(nx[i] - base), lh, __fmul_rn(lh, a1), __fmul_rn(lh, a2));
         }
         __syncthreads();
-        const float tau0 = (float)(im[0].xt - base), tau1 = (float)(im[1].xt - base),
-                    tau2 = (float)(im[2].xt - base);
-        const int s1 = im[1].start, s2 = im[2].start;
-        const int u10 = im[0].U1, u11 = im[1].U1, u12 = im[2].U1;
-        const int u20 = im[0].U2, u21 = im[1].U2, u22 = im[2].U2;
-        float acc = 0.f, cmp = 0.f;
-        for (int k = 0; k < cnt; ++k) {
-            const int jj = t0 + k;
-            const bool g1 = jj >= s1, g2 = jj >= s2;
-            const float tr = g2 ? tau2 : (g1 ? tau1 : tau0);
-            const int U1 = g2 ? u12 : (g1 ? u11 : u10);
-            const int U2 = g2 ? u22 : (g1 ? u21 : u20);
-            const float4 e = sh[k];
-            const float d = tr - e.x;
-            const float y = rsqrt_approx(fmaf(d, d, eps2));
-            const float z = y * y;
-            const float c = z * fmaf(z, e.w, e.z);
-            const float v = (jj < U1) ? -c : ((jj >= U2) ? c : e.y * (d * y));
-            const float w = v - cmp;
-            const float t = acc + w;
-            cmp = (t - acc) - w;
-            acc = t;
+        if (t0 + kNearTile <= nd.m1) fetch(t0 + kNearTile);
+        float tau[2] = {0.f, 0.f};
+        const int s0 = near_side(im[0], t0, cnt, base, tau[0]), s1 = near_side(im[1], t0, cnt, base, tau[1]);
+        const bool far = __all_sync(0xffffffffu, (s0 == 1 || s0 == 2) && (s1 == 1 || s1 == 2));
+        const bool near = __all_sync(0xffffffffu, s0 == 3 && s1 == 3);
+        const float2 e2v = make_float2(eps2, eps2), m1 = make_float2(-1.f, -1.f);
+        const float2 tau2 = make_float2(tau[0], tau[1]);
+        float2 acc = make_float2(0.f, 0.f), nc = make_float2(0.f, 0.f);
+        const float4* tile = sh[buf];
+        if (far) {
+            const float2 sgn = make_float2(s0 == 1 ? -1.f : 1.f, s1 == 1 ? -1.f : 1.f);
+#pragma unroll 4
+            for (int k = 0; k < cnt; ++k) {
+                const float4 e = tile[k];
+                const float2 d = __ffma2_rn(make_float2(e.x, e.x), m1, tau2);
+                const float2 r2 = __ffma2_rn(d, d, e2v);
+                const float2 y = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+                const float2 z = __fmul2_rn(y, y);
+                const float2 c = __fmul2_rn(z, __ffma2_rn(z, make_float2(e.w, e.w), make_float2(e.z, e.z)));
+                const float2 w = __ffma2_rn(c, sgn, nc);  // +-c, exactly, less the compensation
+                const float2 t = __fadd2_rn(acc, w);
+                nc = __ffma2_rn(__ffma2_rn(acc, m1, t), m1, w);
+                acc = t;
+            }
+        } else if (near) {
+            // 1, in a form that keeps v's own rounding before it meets the compensation
+            const float2 one = make_float2(s0 == 3 ? 1.f : -1.f, s1 == 3 ? 1.f : -1.f);
+#pragma unroll 4
+            for (int k = 0; k < cnt; ++k) {
+                const float4 e = tile[k];
+                const float2 d = __ffma2_rn(make_float2(e.x, e.x), m1, tau2);
+                const float2 r2 = __ffma2_rn(d, d, e2v);
+                const float2 y = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+                const float2 v = __fmul2_rn(make_float2(e.y, e.y), __fmul2_rn(d, y));
+                const float2 w = __ffma2_rn(v, one, nc);
+                const float2 t = __fadd2_rn(acc, w);
+                nc = __ffma2_rn(__ffma2_rn(acc, m1, t), m1, w);
+                acc = t;
+            }
+        } else {
+            near_mixed(im[0], t0, cnt, base, tile, eps2, acc.x, nc.x);
+            near_mixed(im[1], t0, cnt, base, tile, eps2, acc.y, nc.y);
         }
-        fp += (double)acc - (double)cmp;
+        fp[0] += (double)acc.x + (double)nc.x;
+        fp[1] += (double)acc.y + (double)nc.y;
     }
+    __syncthreads();  // the next leaf reuses shared memory
 }
 
 struct NearArgs {
@@ -673,10 +770,18 @@ struct NearArgs {
     double L, eps, cbg, norm;
     Stage S;
     int* err;
+    // shared near lists: `parts` CTAs take a part each and leave their sums in
+    // part[p * n + j] for k_near_add
+    int parts, n;
+    double* part;
 };
 
-// Near field of target block yb of leaf l (all threads of the CTA together).
-__device__ void near_item(const NearArgs& A, int l, int yb, float4* shg, float2 (*shb)[kNearTile]) {
+// Near field of target block yb of leaf l from part `part` of its near list,
+// pairs of targets h0 .. h0 + kPairs - 1 of each thread's kNearR (all threads of
+// the CTA together).
+template <int kPairs>
+__device__ void near_item(const NearArgs& A, int l, int yb, int h0, int part, float4 (*shg)[kNearTile],
+                          float2 (*shb)[kNearTile]) {
     const TNode* __restrict__ nodes = A.nodes;
     const int* __restrict__ near_list = A.near_list;
     const double* __restrict__ sx = A.sx;
@@ -692,30 +797,44 @@ __device__ void near_item(const NearArgs& A, int l, int yb, float4* shg, float2 
     const double band = kNearBand * eps;
     const double e2d = eps * eps;
     const float eps2 = (float)e2d, a1 = (float)(e2d / 2), a2 = (float)(e2d * e2d / 8);
-    int jt[kNearR];
-    double x[kNearR], exact[kNearR], fp[kNearR];
+    if (tb0 + 2 * h0 * kNearThreads > leaf.m1) return;  // none of these targets is real
+    double x[kNearR], exact[2 * kPairs], fp[2 * kPairs];
 #pragma unroll
     for (int r = 0; r < kNearR; ++r) {
-        jt[r] = tb0 + threadIdx.x + r * kNearThreads;
-        x[r] = (jt[r] <= leaf.m1) ? sx[jt[r]] : sx[leaf.m0];  // padded targets repeat a real one
-        exact[r] = 0.0;
-        fp[r] = 0.0;
+        const int j = tb0 + threadIdx.x + r * kNearThreads;
+        x[r] = (j <= leaf.m1) ? sx[j] : sx[leaf.m0];  // padded targets repeat a real one
     }
-    for (int q = 0; q < A.near_n[l]; ++q) {
+#pragma unroll
+    for (int r = 0; r < 2 * kPairs; ++r) exact[r] = fp[r] = 0.0;
+    double xp[kPairs][2];  // this CTA's targets
+#pragma unroll
+    for (int h = 0; h < kPairs; ++h) {
+        xp[h][0] = kPairs == kNearR / 2 ? x[2 * h] : (h0 ? x[2] : x[0]);
+        xp[h][1] = kPairs == kNearR / 2 ? x[2 * h + 1] : (h0 ? x[3] : x[1]);
+    }
+    const int nn = A.near_n[l], q0 = nn * part / A.parts, q1 = nn * (part + 1) / A.parts;
+    for (int q = q0; q < q1; ++q) {
         const TNode nd = nodes[near_list[(size_t)l * kNearCap + q]];
         const double xlo = sx[nd.m0], xhi = sx[nd.m1];
-        double xt[kNearR];
+        // decided for all targets of the block, whichever of them this CTA takes
+        double xtr[kNearR];
         bool simple = true;
 #pragma unroll
         for (int r = 0; r < kNearR; ++r) {
             const double m = round((x[r] - xlo) / L);
-            xt[r] = x[r] - m * L;
-            simple = simple && (round((x[r] - xhi) / L) == m) && (xlo >= xt[r] - band) && (xhi <= xt[r] + band);
+            xtr[r] = x[r] - m * L;
+            simple = simple && (round((x[r] - xhi) / L) == m) && (xlo >= xtr[r] - band) && (xhi <= xtr[r] + band);
         }
         if (__syncthreads_and(simple)) {
+            double xt[2 * kPairs];
+#pragma unroll
+            for (int h = 0; h < kPairs; ++h) {
+                xt[2 * h] = kPairs == kNearR / 2 ? xtr[2 * h] : (h0 ? xtr[2] : xtr[0]);
+                xt[2 * h + 1] = kPairs == kNearR / 2 ? xtr[2 * h + 1] : (h0 ? xtr[3] : xtr[1]);
+            }
             const double sl = range_sum(pl, nd.m0, nd.m1 + 1), slx = range_sum(plx, nd.m0, nd.m1 + 1);
 #pragma unroll
-            for (int r = 0; r < kNearR; ++r) exact[r] -= cbg * (xt[r] * sl - slx);
+            for (int r = 0; r < 2 * kPairs; ++r) exact[r] -= cbg * (xt[r] * sl - slx);
             const float2 e2v = make_float2(eps2, eps2), m1 = make_float2(-1.f, -1.f);
             // software pipeline: each thread holds two sources of the next tile
             // in registers while the current tile is computed; one barrier per tile
@@ -745,9 +864,9 @@ __device__ void near_item(const NearArgs& A, int l, int yb, float4* shg, float2 
                 }
                 __syncthreads();
                 if (t0 + kNearTile <= nd.m1) fetch(t0 + kNearTile);
-                float2 tau2[kNearR / 2], acc2[kNearR / 2], ncmp2[kNearR / 2];
+                float2 tau2[kPairs], acc2[kPairs], ncmp2[kPairs];
 #pragma unroll
-                for (int h = 0; h < kNearR / 2; ++h) {
+                for (int h = 0; h < kPairs; ++h) {
                     tau2[h] = make_float2((float)(xt[2 * h] - base), (float)(xt[2 * h + 1] - base));
                     acc2[h] = make_float2(0.f, 0.f);
                     ncmp2[h] = make_float2(0.f, 0.f);
@@ -762,7 +881,7 @@ __device__ void near_item(const NearArgs& A, int l, int yb, float4* shg, float2 
                         const float2 sx2 = u ? make_float2(e4.z, e4.z) : make_float2(e4.x, e4.x);
                         const float2 qh = u ? make_float2(e4.w, e4.w) : make_float2(e4.y, e4.y);
 #pragma unroll
-                        for (int h = 0; h < kNearR / 2; ++h) {
+                        for (int h = 0; h < kPairs; ++h) {
                             // differences as FMAs with -1 (exact products): no sign
                             // flips; Kahan with the negated compensation nc = -c
                             const float2 d = __ffma2_rn(sx2, m1, tau2[h]);
@@ -778,7 +897,7 @@ __device__ void near_item(const NearArgs& A, int l, int yb, float4* shg, float2 
                     }
                 }
 #pragma unroll
-                for (int h = 0; h < kNearR / 2; ++h) {
+                for (int h = 0; h < kPairs; ++h) {
                     fp[2 * h] += (double)acc2[h].x + (double)ncmp2[h].x;
                     fp[2 * h + 1] += (double)acc2[h].y + (double)ncmp2[h].y;
                 }
@@ -786,66 +905,37 @@ __device__ void near_item(const NearArgs& A, int l, int yb, float4* shg, float2 
             __syncthreads();  // the general path and the next leaf reuse shared memory
         } else {
 #pragma unroll 1
-            for (int r = 0; r < kNearR; ++r)
-                near_general(nd, x[r], sx, lam, pl, plx, L, band, cbg, eps2, a1, a2, shg, exact[r], fp[r], err);
+            for (int h = 0; h < kPairs; ++h)
+                near_general2(nd, xp[h], sx, lam, pl, plx, L, band, cbg, eps2, a1, a2, shg, exact + 2 * h, fp + 2 * h,
+                              err);
         }
     }
 #pragma unroll
-    for (int r = 0; r < kNearR; ++r)
-        if (jt[r] <= leaf.m1) apply_stage(A.S, A.sidx[jt[r]], A.efar[jt[r]] + A.norm * (exact[r] + fp[r]));
+    for (int r = 0; r < 2 * kPairs; ++r) {
+        const int j = tb0 + threadIdx.x + (2 * h0 + r) * kNearThreads;
+        if (j > leaf.m1) continue;
+        if (A.parts > 1) A.part[(size_t)part * A.n + j] = exact[r] + fp[r];
+        else apply_stage(A.S, A.sidx[j], A.efar[j] + A.norm * (exact[r] + fp[r]));
+    }
 }
 
-// One CTA per (leaf, target block): grid (leaf capacity, blocks per leaf).
+// The parts of shared near lists, in part order, and the stage epilogue.
+__global__ void k_near_add(NearArgs A) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= A.n || A.meta[2]) return;
+    double s = A.part[j];
+    for (int p = 1; p < A.parts; ++p) s += A.part[(size_t)p * A.n + j];
+    apply_stage(A.S, A.sidx[j], A.efar[j] + A.norm * s);
+}
+
+// One CTA per (leaf, target block, group of kPairs pairs of targets and part of
+// the near list).
+template <int kPairs>
 __global__ void __launch_bounds__(kNearThreads) k_near32(NearArgs A) {
-    __shared__ float4 shg[kNearTile];          // general path: {s, lambda/2, lambda/2 a1, lambda/2 a2}
+    __shared__ float4 shg[2][kNearTile];       // general path: {s, lambda/2, lambda/2 a1, lambda/2 a2}
     __shared__ __align__(16) float2 shb[2][kNearTile];  // band path: {s, lambda/2}, double-buffered
-    near_item(A, blockIdx.x, blockIdx.y, shg, shb);
-}
-
-// Work of item i = l * nyb + yb: its targets times the sources of its leaf's
-// near list (0 for items beyond the tree's leaves or their points).
-__global__ void k_near_cost(NearArgs A, int nitems, int nyb, unsigned* __restrict__ cost, int* __restrict__ ids) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    const int l = i / nyb, yb = i - l * nyb;
-    unsigned c = 0;
-    if (l < A.meta[1] && !A.meta[2]) {
-        const TNode leaf = A.nodes[A.leaves[l]];
-        const int tb0 = leaf.m0 + yb * kNearBlock;
-        if (tb0 <= leaf.m1) {
-            const int nt = min(kNearBlock, leaf.m1 - tb0 + 1);
-            long long ns = 0;
-            for (int q = 0; q < A.near_n[l]; ++q) {
-                const TNode nd = A.nodes[A.near_list[(size_t)l * kNearCap + q]];
-                ns += nd.m1 - nd.m0 + 1;
-            }
-            c = (unsigned)min((long long)nt * ns / 64 + 1, (long long)UINT_MAX);
-        }
-    }
-    cost[i] = c;
-    ids[i] = i;
-}
-
-// Persistent: a one-wave grid takes items from an atomic counter in the order
-// `order` gives (most work first), so that the launch does not end on a
-// leaf with a long near list; items of no work come last and are skipped.
-__global__ void __launch_bounds__(kNearThreads) k_near32_persistent(NearArgs A, int nitems, int nyb,
-                                                                     const int* __restrict__ order,
-                                                                     int* __restrict__ counter) {
-    __shared__ float4 shg[kNearTile];
-    __shared__ __align__(16) float2 shb[2][kNearTile];
-    __shared__ int s_item;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const int k = atomicAdd(counter, 1);
-            s_item = k < nitems ? order[k] : -1;
-        }
-        __syncthreads();
-        const int item = s_item;
-        __syncthreads();
-        if (item < 0) break;
-        near_item(A, item / nyb, item % nyb, shg, shb);
-    }
+    constexpr int kGroups = kNearR / 2 / kPairs;
+    near_item<kPairs>(A, blockIdx.x, blockIdx.y, blockIdx.z % kGroups * kPairs, blockIdx.z / kGroups, shg, shb);
 }
 
 __global__ void k_mul(const double* __restrict__ a, const double* __restrict__ b, int n, double* __restrict__ c) {
@@ -1001,32 +1091,21 @@ class Treecode final : public FieldEngine {
             scan_f64_inclusive(lam_.p, pl_.p, n, scan_.p, st);
             k_mul<<<(n + T - 1) / T, T, 0, st>>>(lam_.p, sx_.p, n, lx_.p);
             scan_f64_inclusive(lx_.p, plx_.p, n, scan_.p, st);
+            // CTAs of two targets per thread, near lists shared by `parts` of
+            // them, where CTAs of four would leave SMs idle
+            const bool split = n < kNearSplit * kNearBlock * sm_count();
+            const int parts = split ? std::max(1, std::min(kNearParts, kNearCtas * sm_count() * (kNearBlock / 2) / n)) : 1;
+            if (parts > 1) npart_.ensure((size_t)parts * n);
             const NearArgs A{nodes_.p, meta_.p, leaves_.p, near_.p, near_n_.p, sx_.p, lam_.p, pl_.p, plx_.p, efar_.p,
-                             iout_.p, L_, eps_, cbg_, norm_, stage, err_.p};
-            if (kNearOrder) {
-                // items in decreasing order of work, taken by a one-wave persistent grid
-                const int nitems = cap_leaves * nyb;
-                k_near_cost<<<(nitems + T - 1) / T, T, 0, st>>>(A, nitems, nyb, ncost_.p, nids_.p);
-                size_t tbn = ntmp_.bytes();
-                FS_CUDA(cub::DeviceRadixSort::SortPairsDescending(ntmp_.p, tbn, ncost_.p, ncost_.p + nitems,
-                                                                  nids_.p, nids_.p + nitems, nitems, 0, 32, st));
-                FS_CUDA(cudaMemsetAsync(ncounter_.p, 0, sizeof(int), st));
-                if (!near_grid_) {
-                    int per_sm = 0;
-                    FS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near32_persistent, kNearThreads,
-                                                                          0));
-                    near_grid_ = std::max(1, per_sm) * sm_count();
-                }
-                ProfScope prof("k_near32", st, last_pairs);
-                k_near32_persistent<<<std::min(near_grid_, nitems), kNearThreads, 0, st>>>(A, nitems, nyb,
-                                                                                          nids_.p + nitems,
-                                                                                          ncounter_.p);
-                FS_LAUNCHED(13);
-            } else {
-                ProfScope prof("k_near32", st, last_pairs);
-                k_near32<<<dim3(cap_leaves, nyb), kNearThreads, 0, st>>>(A);
-                FS_LAUNCHED(12);
+                             iout_.p, L_, eps_, cbg_, norm_, stage, err_.p, parts, n, npart_.p};
+            ProfScope prof("k_near32", st, last_pairs);
+            if (split) k_near32<1><<<dim3(cap_leaves, nyb, 2 * parts), kNearThreads, 0, st>>>(A);
+            else k_near32<2><<<dim3(cap_leaves, nyb), kNearThreads, 0, st>>>(A);
+            if (parts > 1) {
+                k_near_add<<<(n + T - 1) / T, T, 0, st>>>(A);
+                FS_LAUNCHED(1);
             }
+            FS_LAUNCHED(12);
         }
     }
 
@@ -1055,14 +1134,6 @@ class Treecode final : public FieldEngine {
             plx_.ensure(n);
             lx_.ensure(n);
             scan_.ensure(scan_f64_scratch(n));
-            const int nitems = cap_leaves * ((N0_ + kNearBlock - 1) / kNearBlock);
-            ncost_.ensure(2 * (size_t)nitems);
-            nids_.ensure(2 * (size_t)nitems);
-            ncounter_.ensure(1);
-            size_t b = 0;
-            FS_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, b, (const unsigned*)nullptr, (unsigned*)nullptr,
-                                                              (const int*)nullptr, (int*)nullptr, nitems, 0, 32));
-            ntmp_.ensure(std::max<size_t>(b, 1));
         }
         nodes_.ensure(cap_nodes);
         leaves_.ensure(cap_leaves);
@@ -1095,11 +1166,7 @@ class Treecode final : public FieldEngine {
     double norm_ = 1, cbg_ = 0;
     DevBuf<uint64_t> kin_, kout_;
     DevBuf<int> iin_, iout_, leaf_of_, leaves_, meta_, far_, far_n_, near_, near_n_, counts_, item_start_, err_;
-    DevBuf<double> sx_, lam_, efar_, mpart_, mom_, consts_, pl_, plx_, lx_, work_, scan_;
-    DevBuf<unsigned> ncost_;
-    DevBuf<int> nids_, ncounter_;
-    DevBuf<unsigned char> ntmp_;
-    int near_grid_ = 0;
+    DevBuf<double> npart_, sx_, lam_, efar_, mpart_, mom_, consts_, pl_, plx_, lx_, work_, scan_;
     int cap_leaves_ = 0;
     DevBuf<TNode> nodes_;
     TreeCells cells_;
