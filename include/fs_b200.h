@@ -38,8 +38,9 @@ typedef enum fs_status {
 
 /* Field solver kind.  DIRECT64 is the reference arithmetic in FP64 (bit-exact
  * with E_MQ_DirectSum); DIRECT32C is held to 1e-6: FP64 cell expansions where
- * 32 epsilon < L <= 5120 epsilon, else the FP32 pair kernel with compensation and
- * FP64 background (the E a session hands out and batches always take the latter); TREECODE64 / TREECODE32C are the barycentric Lagrange
+ * 32 epsilon < L <= 5120 epsilon and n L / epsilon >= 2e7 (n sources), else FP32
+ * pair kernels with compensation and FP64 background (the E a session hands out
+ * and batches always take the latter); TREECODE64 / TREECODE32C are the barycentric Lagrange
  * treecode of E_MQ_Treecode with an FP64 / FP32-compensated near field;
  * DIRECT64_OPEN is E_MQ_DirectSum_openbcs (src/FieldStructure.cpp:170-192),
  * open boundaries, bit-exact, field plugin only (L is ignored). */

@@ -15,9 +15,8 @@
 // O(N) work for the points and (cells x 16)-sized pair sums between them,
 // where the pairwise sum is O(N^2): at 525,825 points of the two-stream box
 // (2,528 cells) one evaluation takes 4e7 FP64 pair terms in place of 2.8e11,
-// 84 us in place of 42.1 ms by the pairwise kernel, and 61 us in place of 170
-// at 2,145 points (both are chains of short launches there).  Its error there
-// is 1e-15 and 1e-14 of E, the pairwise kernel's 1e-11 and 2e-10.
+// 84 us in place of 42.1 ms by the pairwise kernel.  Its error there is 1e-15 of
+// E, the pairwise kernel's 1e-11.
 //
 // The pair sums run on two levels.  16 cells form a group; the near groups
 // (-1, 0, +1) and the group half a period away, whose pairs change their

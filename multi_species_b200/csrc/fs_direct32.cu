@@ -88,16 +88,24 @@ __device__ __forceinline__ double band_acc64(double q4, double d, double r, doub
 
 // x -> [0, L) and its order-preserving key (non-negative doubles sort as
 // unsigned integers).
+__device__ __forceinline__ uint64_t wrap_key(double x, double L) {
+    double w = x - L * floor(x / L);
+    if (w >= L) w -= L;
+    if (w < 0.0) w = 0.0;
+    w = w + 0.0;  // -0 -> +0
+    return (uint64_t)__double_as_longlong(w);
+}
 __global__ void k_wrap_keys(const double* __restrict__ x, int n, double L, uint64_t* __restrict__ keys,
                             int* __restrict__ idx) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double w = x[i] - L * floor(x[i] / L);
-    if (w >= L) w -= L;
-    if (w < 0.0) w = 0.0;
-    w = w + 0.0;  // -0 -> +0
-    keys[i] = (uint64_t)__double_as_longlong(w);
+    keys[i] = wrap_key(x[i], L);
     idx[i] = i;
+}
+
+__device__ __forceinline__ float4 source_record(double s, double q, double a1, double a2) {
+    const float qh = (float)(0.5 * q);
+    return make_float4((float)s, qh, (float)((double)qh * a1), (float)((double)qh * a2));
 }
 
 // Sorted sources -> tile-relative FP32 records {s, q/2, q/2 a1, q/2 a2}
@@ -119,8 +127,7 @@ __global__ void k_gather_sources(const uint64_t* __restrict__ skeys, const int* 
     const double base = key_to_x(skeys[(j / kS) * kS]);
     if (j % kS == 0) tbase[j / kS] = base;
     const double qj = q[sidx[j]];
-    const float qh = (float)(0.5 * qj);
-    src[j] = make_float4((float)(xj - base), qh, (float)((double)qh * a1), (float)((double)qh * a2));
+    src[j] = source_record(xj - base, qj, a1, a2);
     src64[j] = make_double2(xj, 0.25 * qj);
     qs[j] = qj;
     qx[j] = qj * xj;
@@ -148,23 +155,13 @@ __device__ __forceinline__ double unrolled_prefix(const double* __restrict__ inc
     return k * incl[n - 1] + (r ? incl[r - 1] : 0.0);
 }
 
-// Per sorted target: the image split J, the near band [U1, U2) in unrolled
-// index space (|d| <= band), and the far-band sign sum.
-__global__ void k_target_info(const uint64_t* __restrict__ tkeys, int nt, int nt_pad,
-                              const uint64_t* __restrict__ skeys, int ns, double L, double band,
-                              const double* __restrict__ pq, TargetInfo* __restrict__ info) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nt_pad) return;
+// The image split J and the near band [U1, U2) in unrolled index space (|d| <=
+// band) of a target at xw.
+__device__ __forceinline__ TargetInfo target_split(double xw, const uint64_t* __restrict__ skeys, int ns, double L,
+                                                   double band) {
     TargetInfo T;
     T.pad = 0;
-    if (i >= nt) {
-        T.tlo = 0.0;
-        T.ffar = 0.0;
-        T.J = T.U1 = T.U2 = 0;
-        info[i] = T;
-        return;
-    }
-    const double xw = key_to_x(tkeys[i]);
+    T.ffar = 0.0;
     const double half = 0.5 * L;
     double th;
     if (xw < half) {
@@ -184,9 +181,34 @@ __global__ void k_target_info(const uint64_t* __restrict__ tkeys, int nt, int nt
     const double c = T.tlo + L;  // d(u) = c - X(u)
     T.U1 = unrolled_lower_bound(skeys, ns, L, T.J, T.J + ns, c - band, false);  // first d <= band
     T.U2 = unrolled_lower_bound(skeys, ns, L, T.U1, T.J + ns, c + band, true);  // first d < -band
+    return T;
+}
+// The exact FP64 sum of sign(d) q/2 beyond the band, from prefix sums.
+__device__ __forceinline__ double far_sign_sum(const TargetInfo& T, const double* __restrict__ pq, int ns) {
     const double p_J = unrolled_prefix(pq, ns, T.J), p_1 = unrolled_prefix(pq, ns, T.U1);
     const double p_2 = unrolled_prefix(pq, ns, T.U2), p_e = unrolled_prefix(pq, ns, T.J + ns);
-    T.ffar = 0.5 * ((p_1 - p_J) - (p_e - p_2));
+    return 0.5 * ((p_1 - p_J) - (p_e - p_2));
+}
+__device__ __forceinline__ TargetInfo no_target() {
+    TargetInfo T;
+    T.pad = 0;
+    T.tlo = T.ffar = 0.0;
+    T.J = T.U1 = T.U2 = 0;
+    return T;
+}
+
+// Per sorted target: split, band and far-band sign sum.
+__global__ void k_target_info(const uint64_t* __restrict__ tkeys, int nt, int nt_pad,
+                              const uint64_t* __restrict__ skeys, int ns, double L, double band,
+                              const double* __restrict__ pq, TargetInfo* __restrict__ info) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nt_pad) return;
+    if (i >= nt) {
+        info[i] = no_target();
+        return;
+    }
+    TargetInfo T = target_split(key_to_x(tkeys[i]), skeys, ns, L, band);
+    T.ffar = far_sign_sum(T, pq, ns);
     info[i] = T;
 }
 
@@ -242,6 +264,7 @@ constexpr bool kStage64 = FS_STAGE64;
 #endif
 constexpr double kBand = FS_PAIR_BAND;  // near band half-width in units of eps
 constexpr int kMaxChunks = 64;
+constexpr double kCellLoad = 2e7;  // n L / epsilon from which sums go through cells (Direct32c::through_cells)
 
 // One (target block, source chunk) of a job: kR targets per thread, the
 // chunk's tiles moved into shared memory by TMA bulk copies on two mbarriers.
@@ -737,7 +760,7 @@ namespace {
 __global__ void k_finalize32(const double* __restrict__ partial, int nchunks, int nt_pad, int nt,
                              const TargetInfo* __restrict__ info, const double* __restrict__ pq,
                              const double* __restrict__ qxsum, int ns, double L, double cbg,
-                             const int* __restrict__ tperm, Stage S) {
+                             const int* __restrict__ tperm, bool form_ffar, Stage S) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nt) return;
     double E = 0.0;
@@ -747,7 +770,7 @@ __global__ void k_finalize32(const double* __restrict__ partial, int nchunks, in
         const double Q = pq[ns - 1];
         const double PJ = (T.J > 0) ? pq[T.J - 1] : 0.0;
         const double B = T.tlo * Q - qxsum[0] + L * (Q - PJ);
-        E += T.ffar;
+        E += form_ffar ? far_sign_sum(T, pq, ns) : T.ffar;
         E -= cbg * B;
     }
     apply_stage(S, tperm[i], E);
@@ -767,6 +790,309 @@ __global__ void k_band_count(int nt, const TargetInfo* __restrict__ info, double
         __syncthreads();
     }
     if (threadIdx.x == 0) atomicAdd(out, sh[0]);
+}
+
+// ---------------------------------------------------------------- few points
+// Up to kSmallMax sources and targets an evaluation is a chain of short launches,
+// so it is made of four: rank sort; source records, prefix sums and target
+// splits; pairs; the final sums.  The order of the sources, the tiles and the
+// path each group of targets takes through a tile are those of the pairwise
+// kernels above, so the FP32 sums are the same; only FP64 sums of tiles are
+// associated differently.  2,145 points without allocation:
+// 171 -> 66 us (pairs 91 -> 21, sort 18 -> 8 us); 8,193 points of a field handle 314
+// -> 130 us; at 16,384 the persistent kernel is as fast.
+constexpr int kSmallMax = 16384;
+constexpr int kRankKeys = 2048;  // keys staged at a time
+
+// Sorted place of every key by counting the keys before it (ties by index, as
+// the stable radix sort leaves them): kParts threads per key, n^2 comparisons,
+// and every CTA forms all keys anew, so a warp per key pays up to a few thousand.
+// Two point sets in one launch: blocks from `split` on take the second.
+template <int kParts>
+__global__ void __launch_bounds__(256) k_rank_sort(const double* __restrict__ xa, int na, uint64_t* __restrict__ ka,
+                                                   int* __restrict__ ia, const double* __restrict__ xb, int nb,
+                                                   uint64_t* __restrict__ kb, int* __restrict__ ib, int split,
+                                                   double L, int* __restrict__ err) {
+    __shared__ uint64_t sh[kRankKeys];
+    if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
+    const bool second = (int)blockIdx.x >= split;
+    const double* __restrict__ x = second ? xb : xa;
+    const int n = second ? nb : na;
+    const int i = ((int)blockIdx.x - (second ? split : 0)) * (256 / kParts) + threadIdx.x / kParts;
+    const int part = threadIdx.x % kParts;
+    constexpr uint64_t kMag = 0x7fffffffffffffffull;  // the bits the radix sort looks at
+    const uint64_t own = i < n ? wrap_key(x[i], L) : 0;
+    int before = 0;
+    for (int base = 0; base < n; base += kRankKeys) {
+        const int cnt = min(kRankKeys, n - base);
+        __syncthreads();
+        for (int k = threadIdx.x; k < cnt; k += 256) sh[k] = wrap_key(x[base + k], L) & kMag;
+        __syncthreads();
+#pragma unroll 4
+        for (int k = part; k < cnt; k += kParts) {
+            const uint64_t v = sh[k];
+            before += v < (own & kMag) || (v == (own & kMag) && base + k < i);
+        }
+    }
+#pragma unroll
+    for (int o = kParts / 2; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (part == 0 && i < n) {
+        (second ? kb : ka)[before] = own;
+        (second ? ib : ia)[before] = i;
+    }
+}
+
+// Block 0: source records, tile bases, inclusive prefix sums of q and the sum of
+// q x (runs of consecutive sources per thread, then a scan over the threads).
+// The other blocks: splits and bands of 128 targets each, the keys searched in
+// shared memory.
+__global__ void __launch_bounds__(1024) k_small_setup(const uint64_t* __restrict__ skeys, const int* __restrict__ sidx,
+                                                      const double* __restrict__ q, int ns, int ns_pad, double a1,
+                                                      double a2, float4* __restrict__ src, double2* __restrict__ src64,
+                                                      double* __restrict__ tbase, double* __restrict__ pq,
+                                                      double* __restrict__ qxsum, const uint64_t* __restrict__ tkeys,
+                                                      int nt, int nt_pad, double L, double band,
+                                                      TargetInfo* __restrict__ info) {
+    extern __shared__ uint64_t sm_keys[];
+    const int t = threadIdx.x;
+    if (blockIdx.x > 0) {
+        for (int k = t; k < ns; k += 1024) sm_keys[k] = skeys[k];
+        __syncthreads();
+        const int i = ((int)blockIdx.x - 1) * 128 + t;
+        if (t < 128 && i < nt_pad)
+            info[i] = i < nt ? target_split(key_to_x(tkeys[i]), sm_keys, ns, L, band) : no_target();
+        return;
+    }
+    __shared__ double wq[32], wx[32];
+    constexpr int kRun = kSmallMax / 1024;
+    const int lane = t & 31, warp = t >> 5, run = (ns_pad + 1023) / 1024, j0 = t * run;
+    double qv[kRun], sq = 0.0, sx = 0.0;
+#pragma unroll
+    for (int k = 0; k < kRun; ++k) {
+        const int j = j0 + k;
+        qv[k] = 0.0;
+        if (k < run && j < ns_pad) {
+            if (j < ns) {
+                const double xj = key_to_x(skeys[j]), base = key_to_x(skeys[j / kS * kS]), qj = q[sidx[j]];
+                if (j % kS == 0) tbase[j / kS] = base;
+                src[j] = source_record(xj - base, qj, a1, a2);
+                src64[j] = make_double2(xj, 0.25 * qj);
+                qv[k] = qj;
+                sq += qj;
+                sx += qj * xj;
+            } else {
+                src[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                src64[j] = make_double2(0.0, 0.0);
+            }
+        }
+    }
+    double inc = sq;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sx += __shfl_xor_sync(0xffffffffu, sx, o);
+    if (lane == 31) {
+        wq[warp] = inc;
+        wx[warp] = sx;
+    }
+    __syncthreads();
+    double before = 0.0;
+    for (int w = 0; w < warp; ++w) before += wq[w];
+    double ex = __shfl_up_sync(0xffffffffu, inc, 1);
+    before += lane ? ex : 0.0;
+#pragma unroll
+    for (int k = 0; k < kRun; ++k) {
+        before += qv[k];
+        if (k < run && j0 + k < ns) pq[j0 + k] = before;
+    }
+    if (t == 0) {
+        double s = 0.0;
+        for (int w = 0; w < 32; ++w) s += wx[w];
+        qxsum[0] = s;
+    }
+}
+
+// One (group of kG targets, tile) per CTA, one target per thread.  kG is the
+// number of targets that choose a tile's path together in the kernel this stands
+// in for (32 times its targets per thread).  There two targets 32 apart share a
+// reciprocal, so each thread forms its partner's r too.
+template <int kG>
+__global__ void __launch_bounds__(kG) k_pairs32_small(PairJob Jb, int* __restrict__ err) {
+    __shared__ __align__(128) float4 tile[kS];
+    __shared__ __align__(128) double2 tile64[kS];
+    __shared__ __align__(8) uint64_t bar;
+    const int tid = threadIdx.x, i = blockIdx.x * kG + tid, t = blockIdx.y;
+    constexpr uint32_t kBytes = kS * sizeof(float4), kBytes64 = kS * sizeof(double2);
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        fence_proxy_async();
+        mbar_expect_tx(&bar, kBytes + kBytes64);
+        bulk_load(tile, Jb.src + (size_t)t * kS, kBytes, &bar);
+        bulk_load(tile64, Jb.src64 + (size_t)t * kS, kBytes64, &bar);
+    }
+    const TargetInfo T = Jb.info[i], To = Jb.info[i ^ 32];
+    const double base = Jb.tbase[t];
+    const int ns = Jb.ns, jlo = t * kS, jend = min(jlo + kS, ns);
+    const double L = Jb.L;
+    __syncthreads();
+    const bool ok = mbar_wait_bounded(&bar, 0, g_mbar_polls);
+    if (!__syncthreads_and(ok)) {
+        if (tid == 0) {
+            atomicExch(err, (int)FS_ERR_TIMEOUT);
+            (void)mbar_wait_bounded(&bar, 0, kMbarPolls);  // the copies land before the CTA exits
+        }
+        return;
+    }
+    float tau = (float)(T.tlo - base);
+    const float tauh = (float)(T.tlo - base + L);
+    const float taul = tau;
+    float sg = 0.f;
+    bool inband = false;
+    if (jend <= T.J) {          // whole tile on the lo image: u = j + n
+        if (jend + ns <= T.U1) sg = 1.f;
+        else if (jlo + ns >= T.U2) sg = -1.f;
+        inband = (jlo + ns >= T.U1) && (jend + ns <= T.U2);
+    } else if (jlo >= T.J) {    // whole tile on the hi image: u = j
+        tau = tauh;
+        if (jend <= T.U1) sg = 1.f;
+        else if (jlo >= T.U2) sg = -1.f;
+        inband = (jlo >= T.U1) && (jend <= T.U2);
+    }
+    const bool careful = __syncthreads_or(sg == 0.f);
+    double acc64 = 0.0;
+    if (!careful) {
+        const float tauo = (float)(jend <= To.J ? To.tlo - base : To.tlo - base + L);
+        const float e2 = Jb.e2f;
+        float acc = 0.f;
+#pragma unroll 8
+        for (int j = 0; j < kS; ++j) {
+            const float4 e = tile[j];
+            const float d = __fsub_rn(tau, e.x), o = __fsub_rn(tauo, e.x);
+            const float r = fmaf(d, d, e2), ro = fmaf(o, o, e2);
+            acc = fmaf(ro, __fmul_rn(e.z, rcp_approx(__fmul_rn(r, ro))), acc);
+        }
+        acc64 -= (double)sg * (double)acc;
+    } else if (__syncthreads_and(inband)) {
+        const double X = (jend <= T.J) ? T.tlo : T.tlo + L, e2d = Jb.eps2d;
+#pragma unroll 8
+        for (int j = 0; j < kS; ++j) {
+            const double2 e = tile64[j];
+            const double d = X - e.x;
+            acc64 = band_acc64(e.y, d, fma(d, d, e2d), acc64);
+        }
+    } else {
+        // the target's band in the tile, by image: sources [b0, b1) on the hi
+        // image (u = j), [c0, c1) on the lo one (u = j + n)
+        const double Xh = T.tlo + L, e2d = Jb.eps2d;
+        const float eps2 = Jb.eps2, a1 = Jb.a1, a2 = Jb.a2;
+        const int b0 = max(T.U1, T.J) - jlo, b1 = min(T.U2, ns) - jlo;
+        const int c0 = T.U1 - ns - jlo, c1 = min(T.U2 - ns, T.J) - jlo;
+        auto in_band = [&](int j) { return (j >= b0 && j < b1) || (j >= c0 && j < c1); };
+        constexpr int kStep = 8;
+        float acc = 0.f, cmp = 0.f;
+        for (int g = 0; g < kS; g += kStep) {
+            // most groups are of one image and one side for the whole warp
+            const int j0 = jlo + g;
+            const bool lo_all = j0 + kStep <= T.J, one = lo_all || j0 >= T.J;
+            const int u0 = lo_all ? j0 + ns : j0;
+            const bool left = u0 + kStep <= T.U1, right = u0 >= T.U2;
+            if (__all_sync(0xffffffffu, one && (left || right))) {
+                const float tg = lo_all ? taul : tauh, sgn = left ? -1.f : 1.f;
+#pragma unroll
+                for (int k = 0; k < kStep; ++k) {
+                    const float4 e = tile[g + k];
+                    const float d = tg - e.x;
+                    const float y = rsqrt_approx(fmaf(d, d, eps2));
+                    const float z = __fmul_rn(y, y);
+                    const float c = __fmul_rn(z, fmaf(z, a2, a1));
+                    const float v = fmaf(__fmul_rn(e.y, sgn), c, -cmp);
+                    const float sum = __fadd_rn(acc, v);
+                    cmp = __fsub_rn(__fsub_rn(sum, acc), v);
+                    acc = sum;
+                }
+                continue;
+            }
+            if (__all_sync(0xffffffffu, one && u0 >= T.U1 && u0 + kStep <= T.U2)) {
+                const double X = lo_all ? T.tlo : Xh;
+#pragma unroll
+                for (int k = 0; k < kStep; ++k) {
+                    const double2 e = tile64[g + k];
+                    const double d = X - e.x;
+                    acc64 = band_acc64(e.y, d, fma(d, d, e2d), acc64);
+                }
+                continue;
+            }
+            // far pairs in FP32 and order, band pairs in FP64
+#pragma unroll
+            for (int k = 0; k < kStep; ++k) {
+                const int j = g + k, idx = jlo + j;
+                const bool lo_img = idx < T.J, band = in_band(j);
+                const float4 e = tile[j];
+                const float d = (lo_img ? taul : tauh) - e.x;
+                const float y = rsqrt_approx(fmaf(d, d, eps2));
+                const float z = __fmul_rn(y, y);
+                const float c = __fmul_rn(z, fmaf(z, a2, a1));
+                const float val = ((lo_img ? idx + ns : idx) < T.U1) ? -c : c;
+                const float v = fmaf(e.y, val, -cmp);
+                const float sum = __fadd_rn(acc, v);
+                const float rest = __fsub_rn(__fsub_rn(sum, acc), v);
+                cmp = band ? cmp : rest;
+                acc = band ? acc : sum;
+                const double2 e64 = tile64[j];
+                const double d64 = (lo_img ? T.tlo : Xh) - e64.x;
+                acc64 = band_acc64(band ? e64.y : 0.0, d64, fma(d64, d64, e2d), acc64);
+            }
+        }
+        acc64 += (double)acc - (double)cmp;
+    }
+    Jb.partial[(size_t)t * Jb.nt_pad + i] = acc64;
+}
+
+// Device scratch of an evaluation of few points.
+struct SmallBuffers {
+    uint64_t *kout, *tkout;  // ns, nt (the same array for a self-field)
+    int *iout, *tiout;
+    float4* src;
+    double2* src64;
+    double *tbase, *pq, *qxsum, *partial;
+    TargetInfo* info;
+};
+
+// `group`: 128 or 256 targets choose a tile's path together; clear_err: *err is
+// set to 0 first.
+void small_field(const SmallBuffers& B, double L, double eps, const double* d_t, int nt, const double* d_s,
+                 const double* d_q, int ns, int nt_pad, int group, const Stage& S, int* err, bool clear_err,
+                 cudaStream_t st) {
+    const bool same = d_t == d_s && nt == ns;
+    const double e2 = eps * eps;
+    const int ntiles = (ns + kS - 1) / kS;
+    const bool warps = std::max(nt, ns) <= 4096;
+    const int per = 256 / (warps ? 32 : 8), sblocks = (ns + per - 1) / per, tblocks = same ? 0 : (nt + per - 1) / per;
+    (warps ? k_rank_sort<32> : k_rank_sort<8>)<<<sblocks + tblocks, 256, 0, st>>>(
+        d_s, ns, B.kout, B.iout, d_t, nt, B.tkout, B.tiout, sblocks, L, clear_err ? err : nullptr);
+    const size_t smem = sizeof(uint64_t) * (size_t)ns;
+    if (smem > 32 * 1024)
+        FS_CUDA(cudaFuncSetAttribute(k_small_setup, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(uint64_t) * kSmallMax)));
+    k_small_setup<<<1 + (nt_pad + 127) / 128, 1024, smem, st>>>(B.kout, B.iout, d_q, ns, ntiles * kS, e2 / 2,
+                                                                e2 * e2 / 8, B.src, B.src64, B.tbase, B.pq, B.qxsum,
+                                                                B.tkout, nt, nt_pad, L, kBand * eps, B.info);
+    const PairJob job{B.src, B.src64, B.tbase, B.info, B.partial, ns, ntiles, 1, nt_pad, L, (float)e2,
+                      (float)(e2 / 2), (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, nt};
+    {
+        ProfScope prof("k_pairs32", st, (double)nt * (double)ns);
+        const dim3 grid((nt + group - 1) / group, ntiles);
+        if (group == 128) k_pairs32_small<128><<<grid, 128, 0, st>>>(job, err);
+        else k_pairs32_small<256><<<grid, 256, 0, st>>>(job, err);
+    }
+    const double cbg = 1 / std::sqrt(L * L + 4 * eps * eps);
+    k_finalize32<<<(nt + 127) / 128, 128, 0, st>>>(B.partial, ntiles, nt_pad, nt, B.info, B.pq, B.qxsum, ns, L, cbg,
+                                                   B.tiout, true, S);
+    FS_LAUNCHED(4);
 }
 
 class Direct32c final : public FieldEngine {
@@ -794,12 +1120,24 @@ class Direct32c final : public FieldEngine {
 
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns, const Stage& stage,
               cudaStream_t st, bool pairwise) override {
-        if (cells_ && !pairwise && nt > 0 && ns > 0) {
+        if (!pairwise && nt > 0 && through_cells(ns)) {
             last_pairs = (double)nt * (double)ns;
             last_nt_ = 0;
             fin_ = Fin{};
             reserve_cells(ns);
             cell_field(plan_, buf_, d_t, nt, d_s, d_q, ns, stage, err_.p, st);
+            return;
+        }
+        if (nt > 0 && ns > 0 && nt <= kSmallMax && ns <= kSmallMax && (R_ == 4 || R_ == 8)) {
+            last_pairs = (double)nt * (double)ns;
+            last_nt_ = nt;
+            fin_ = Fin{};
+            const bool same = d_t == d_s && nt == ns;
+            const int ntiles = (ns + kS - 1) / kS, nt_pad = (nt + kTBPad - 1) / kTBPad * kTBPad;
+            reserve(ns, ntiles * kS, same ? 0 : nt, nt_pad, (size_t)ntiles * nt_pad, ntiles);
+            const SmallBuffers B{kout_.p, same ? kout_.p : tkout_.p, iout_.p, same ? iout_.p : tiout_.p, src_.p,
+                                 src64_.p, tbase_.p, pq_.p, qxsum_.p, partial_.p, info_.p};
+            small_field(B, L_, eps_, d_t, nt, d_s, d_q, ns, nt_pad, 32 * R_, stage, err_.p, false, st);
             return;
         }
         // a standalone launch: one persistent wave over about 32 items per CTA
@@ -889,12 +1227,18 @@ class Direct32c final : public FieldEngine {
         fin_.pending = false;
         const int T = 256;
         k_finalize32<<<(fin_.nt + T - 1) / T, T, 0, st>>>(partial_.p, fin_.nchunks, fin_.nt_pad, fin_.nt, info_.p,
-                                                           pq_.p, qxsum_.p, fin_.ns, L_, cbg_, fin_.tperm, fin_.stage);
+                                                           pq_.p, qxsum_.p, fin_.ns, L_, cbg_, fin_.tperm, false, fin_.stage);
         FS_LAUNCHED(1);
     }
 
     int* error_flag() override { return err_.p; }
-    bool has_cells() const override { return cells_; }
+    // The two forms of the sum agree to the pairwise one's FP32 error: 2e-10 of E
+    // at L = 250 epsilon whatever n, falling as epsilon / L, and more for few
+    // points (1e-9 at 600).  Cells take over where that leaves E within a few
+    // 1e-10 of the pairwise sum (n L / epsilon from 2e7: 80,000 points of a Landau
+    // box, 13,000 of the two-stream box), which is also where they are faster by
+    // more than the launches.
+    bool through_cells(int n) const override { return cells_ && n * (L_ / eps_) >= kCellLoad; }
 
     // Pairs of the last evaluation; while profiling, after a pairwise one, also
     // the band pairs among them, recorded as "pairs32_band_pairs".
@@ -1166,7 +1510,7 @@ void direct32c_noalloc(double L, double eps, double* d_es, const double* d_x, co
     S.kind = STAGE_STORE;
     S.out = d_es;
     CellPlan plan;
-    if (cell_plan(L, eps, &plan)) {
+    if (n * (L / eps) >= kCellLoad && cell_plan(L, eps, &plan)) {
         CellBuffers B;
         B.kin = reinterpret_cast<uint32_t*>(at(kNoAllocCells.keys));
         B.kout = B.kin + kNoAllocMaxPoints;
@@ -1210,6 +1554,12 @@ void direct32c_noalloc(double L, double eps, double* d_es, const double* d_x, co
     const int ns_pad = ntiles * kS;
     constexpr int R = 4;
     const int nt_pad = (n + kTBPad - 1) / kTBPad * kTBPad;
+    if (n <= kSmallMax && (size_t)ntiles * nt_pad <= (size_t)kNoAllocMaxChunks * kNoAllocMaxPoints) {
+        const SmallBuffers B{kout, kout, iout, iout, src, src64, tbase, pq, qxsum, partial, info};
+        small_field(B, L, eps, d_x, n, d_x, d_q, n, nt_pad, 32 * R, S, err, true, st);
+        finish(err);
+        return;
+    }
     const int tblocks = nt_pad / (kNT * R);
     const int want = sm_count() * 8 * 4;
     int nchunks = std::min(std::min(ntiles, kNoAllocMaxChunks), std::max(1, (want + tblocks - 1) / tblocks));
@@ -1236,7 +1586,7 @@ void direct32c_noalloc(double L, double eps, double* d_es, const double* d_x, co
                       (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, n};
     launch_pairs(R, dim3(tblocks, nchunks), st, job, err);
     const double cbg = 1 / std::sqrt(L * L + 4 * eps * eps);
-    k_finalize32<<<(n + T - 1) / T, T, 0, st>>>(partial, nchunks, nt_pad, n, info, pq, qxsum, n, L, cbg, iout, S);
+    k_finalize32<<<(n + T - 1) / T, T, 0, st>>>(partial, nchunks, nt_pad, n, info, pq, qxsum, n, L, cbg, iout, false, S);
     FS_LAUNCHED(6);
     finish(err);
 }

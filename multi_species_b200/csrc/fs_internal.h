@@ -252,9 +252,12 @@ class FieldEngine {
     // `pairwise`: by the pairwise kernel where the engine has another form too.
     virtual void eval(const double* d_targets, int nt, const double* d_sources, const double* d_q,
                       int ns, const Stage& stage, cudaStream_t st, bool pairwise = false) = 0;
-    // Whether evaluations that are not `pairwise` go through cells (prepare()
-    // is always pairwise).
-    virtual bool has_cells() const { return false; }
+    // Whether an evaluation of n sources that is not `pairwise` goes through
+    // cells (prepare() is always pairwise).
+    virtual bool through_cells(int n) const {
+        (void)n;
+        return false;
+    }
     // Device int set non-zero by a kernel whose bounded wait gave up (or null).
     virtual int* error_flag() { return nullptr; }
     // Kernel-level evaluations of the last call (pairs for the direct sums;

@@ -1054,7 +1054,7 @@ struct Sim {
     // session to 1e-10, as do positions and velocities, which integrate E.
     // e_stale: the points have moved since e was formed.
     DevBuf<double> ek;
-    bool via_cells = false, e_stale = false;
+    bool cells_wanted = false, via_cells = false, e_stale = false;
     DevBuf<int> status;
     std::unique_ptr<FieldEngine> field;
     cudaStream_t st = nullptr;
@@ -1334,8 +1334,8 @@ struct Sim {
                 break;
             default: fail(FS_ERR_ARG, "unknown field kind");
         }
-        via_cells = cells && field->has_cells();
-        if (via_cells) ek.ensure(N);
+        cells_wanted = cells;
+        choose_form();
         base.x = x.p;
         base.p = p.p;
         base.pst = pst.p;
@@ -1343,6 +1343,13 @@ struct Sim {
         base.accP = accP.p;
         reduced_field();  // AMRSimulation ctor: evaluate_field_uniform_grid(0)
         check_status();
+    }
+
+    // Stage fields through cells or pairwise, by the number of points (a call on
+    // the points uses one form throughout).
+    void choose_form() {
+        via_cells = cells_wanted && field->through_cells(N);
+        if (via_cells) ek.ensure(N);
     }
 
     // direct-equivalent pairs always; kernel-level evaluations when profiling
@@ -1579,7 +1586,7 @@ struct Sim {
         upload(f, af);
         upload(qw, aq);
         for (auto* b : {&e, &xkA, &xkB, &pst, &accX, &accP}) b->ensure(N);
-        if (via_cells) ek.ensure(N);
+        choose_form();
         base.x = x.p;
         base.p = p.p;
         base.pst = pst.p;
@@ -1733,15 +1740,15 @@ struct Sim {
     FieldCall call(int c) const {
         const double t2 = t + prm.dt * 0.5, t4 = t + prm.dt;
         switch (c) {
-            case 0: return with_drive(FieldCall{xkA.p, N, qw.p, stage(STAGE_RK2, xkB.p)}, t2);
-            case 1: return with_drive(FieldCall{xkB.p, N, qw.p, stage(STAGE_RK3, xkA.p)}, t2);
-            case 2: return with_drive(FieldCall{xkA.p, N, qw.p, stage(STAGE_RK4, nullptr)}, t4);
+            case 0: return with_drive(FieldCall{xkA.p, N, qw.p, stage(STAGE_RK2, xkB.p), !via_cells}, t2);
+            case 1: return with_drive(FieldCall{xkB.p, N, qw.p, stage(STAGE_RK3, xkA.p), !via_cells}, t2);
+            case 2: return with_drive(FieldCall{xkA.p, N, qw.p, stage(STAGE_RK4, nullptr), !via_cells}, t4);
             default: {
                 if (remeshing) return reduced_call();
                 Stage S = base;
                 S.kind = STAGE_STORE;
                 S.out = via_cells ? ek.p : e.p;
-                return with_drive(FieldCall{x.p, N, qw.p, S}, t);
+                return with_drive(FieldCall{x.p, N, qw.p, S, !via_cells}, t);
             }
         }
     }
