@@ -1119,8 +1119,8 @@ class Direct32c final : public FieldEngine {
 
 
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns, const Stage& stage,
-              cudaStream_t st, bool pairwise) override {
-        if (!pairwise && nt > 0 && through_cells(ns)) {
+              cudaStream_t st, PairForm form) override {
+        if (form == PairForm::any && nt > 0 && through_cells(ns)) {
             last_pairs = (double)nt * (double)ns;
             last_nt_ = 0;
             fin_ = Fin{};
@@ -1128,7 +1128,7 @@ class Direct32c final : public FieldEngine {
             cell_field(plan_, buf_, d_t, nt, d_s, d_q, ns, stage, err_.p, st);
             return;
         }
-        if (nt > 0 && ns > 0 && nt <= kSmallMax && ns <= kSmallMax && (R_ == 4 || R_ == 8)) {
+        if (form != PairForm::batch && nt > 0 && ns > 0 && nt <= kSmallMax && ns <= kSmallMax && (R_ == 4 || R_ == 8)) {
             last_pairs = (double)nt * (double)ns;
             last_nt_ = nt;
             fin_ = Fin{};

@@ -252,7 +252,7 @@ class Direct64Open final : public FieldEngine {
    public:
     explicit Direct64Open(double eps) : eps_(eps) {}
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns, const Stage& stage,
-              cudaStream_t st, bool) override {
+              cudaStream_t st, PairForm) override {
         last_pairs = (double)nt * (double)ns;
         if (nt <= 0) return;
         const int blocks = (nt + kThreads64 - 1) / kThreads64;
@@ -317,7 +317,7 @@ class Direct64 final : public FieldEngine {
         fast_ = mid(L) && mid(eps) && division_is_product(L, K_.zh, K_.zl);
     }
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns,
-              const Stage& stage, cudaStream_t st, bool) override {
+              const Stage& stage, cudaStream_t st, PairForm) override {
         last_pairs = (double)nt * (double)ns;
         if (nt <= 0) return;
         ProfScope prof("k_direct64", st, last_pairs);

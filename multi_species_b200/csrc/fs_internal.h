@@ -243,17 +243,20 @@ void cell_field(const CellPlan& P, const CellBuffers& B, const double* d_t, int 
                 const double* d_q, int ns, const Stage& S, int* err, cudaStream_t st);
 void set_cell_polls(long long polls);
 
+// How an evaluation's pairs are summed where an engine has several ways: as it
+// sees fit; pair by pair; or pair by pair in the tiles and order that prepare()
+// uses (members of a batch, whose results do not depend on how they started).
+enum class PairForm { any, pairwise, batch };
+
 class FieldEngine {
    public:
     virtual ~FieldEngine() = default;
     // Field at targets from sources (device pointers), result through the
     // stage epilogue, enqueued on `st`.  For targets == sources pass the same
     // pointer and nt == ns.
-    // `pairwise`: by the pairwise kernel where the engine has another form too.
     virtual void eval(const double* d_targets, int nt, const double* d_sources, const double* d_q,
-                      int ns, const Stage& stage, cudaStream_t st, bool pairwise = false) = 0;
-    // Whether an evaluation of n sources that is not `pairwise` goes through
-    // cells (prepare() is always pairwise).
+                      int ns, const Stage& stage, cudaStream_t st, PairForm form = PairForm::any) = 0;
+    // Whether an evaluation of n sources in form `any` goes through cells.
     virtual bool through_cells(int n) const {
         (void)n;
         return false;

@@ -1054,7 +1054,7 @@ struct Sim {
     // session to 1e-10, as do positions and velocities, which integrate E.
     // e_stale: the points have moved since e was formed.
     DevBuf<double> ek;
-    bool cells_wanted = false, via_cells = false, e_stale = false;
+    bool cells_wanted = true, via_cells = false, e_stale = false;
     DevBuf<int> status;
     std::unique_ptr<FieldEngine> field;
     cudaStream_t st = nullptr;
@@ -1192,8 +1192,8 @@ struct Sim {
         done.push_back(device);
     }
 
-    // `cells`: stage fields through cells where the field has them (a batch's
-    // members share pairwise launches instead).
+    // `cells`: a session of its own, whose stage fields go through cells where the
+    // field has them; a batch's members share pairwise launches instead.
     void create(const fs_sim_params& P, cudaStream_t external, bool cells) {
         prm = P;
         if (P.num_species < 1 || P.num_species > 8) fail(FS_ERR_ARG, "num_species must be 1..8");
@@ -1375,7 +1375,8 @@ struct Sim {
     };
 
     void run_call(const FieldCall& fc) {
-        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, fc.pairwise);
+        const PairForm form = !cells_wanted ? PairForm::batch : (fc.pairwise ? PairForm::pairwise : PairForm::any);
+        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, form);
         account();
     }
 
@@ -1386,7 +1387,7 @@ struct Sim {
         S.kind = STAGE_STORE;
         S.out = e.p;
         const FieldCall fc = with_drive(FieldCall{x.p, N, qw.p, S, true}, t);
-        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, true);
+        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, PairForm::pairwise);
         if (profiling_enabled()) (void)field->actual_work(st);
         e_stale = false;
     }

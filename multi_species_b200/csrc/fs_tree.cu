@@ -1179,7 +1179,7 @@ class Treecode final : public FieldEngine {
     }
 
     void eval(const double* d_t, int nt, const double* d_s, const double* d_q, int ns, const Stage& stage,
-              cudaStream_t st, bool) override {
+              cudaStream_t st, PairForm) override {
         (void)d_t;
         if (nt != ns) fail(FS_ERR_ARG, "treecode evaluates at the sources: nt must equal ns");
         last_pairs = (double)ns * (double)ns;
