@@ -33,6 +33,7 @@ struct fs_field {
     std::unique_ptr<fsb::FieldEngine> engine;
     cudaStream_t st = nullptr;
     fsb::DevBuf<double> t, s, q, e;
+    fsb::HostStage stage;
     ~fs_field() {
         if (st) cudaStreamDestroy(st);
     }
@@ -107,18 +108,19 @@ fs_status fs_field_eval(fs_field* field, double* es, const double* targets, int 
         field->q.ensure(std::max(ns, 1));
         field->e.ensure(std::max(nt, 1));
         const bool same = (targets == sources) && nt == ns;
+        std::vector<fsb::HostCopy> in;
         if (ns) {
-            FS_CUDA(cudaMemcpyAsync(field->s.p, sources, sizeof(double) * ns, cudaMemcpyHostToDevice, st));
-            FS_CUDA(cudaMemcpyAsync(field->q.p, q_ws, sizeof(double) * ns, cudaMemcpyHostToDevice, st));
+            in.push_back({field->s.p, sources, sizeof(double) * ns});
+            in.push_back({field->q.p, q_ws, sizeof(double) * ns});
         }
-        if (nt && !same)
-            FS_CUDA(cudaMemcpyAsync(field->t.p, targets, sizeof(double) * nt, cudaMemcpyHostToDevice, st));
+        if (nt && !same) in.push_back({field->t.p, targets, sizeof(double) * nt});
+        field->stage.to_device(in, st);
         fsb::Stage S;
         S.kind = fsb::STAGE_STORE;
         S.out = field->e.p;
         if (nt) {
             field->engine->eval(same ? field->s.p : field->t.p, nt, field->s.p, field->q.p, ns, S, st);
-            FS_CUDA(cudaMemcpyAsync(es, field->e.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
+            field->stage.to_host({{es, field->e.p, sizeof(double) * nt}}, st);
         }
         field->check_errors(st);
     });

@@ -71,6 +71,29 @@ void prof_release(std::vector<ProfNode>& nodes);
 // near pairs and far terms) under `name` while profiling is enabled.
 void prof_add_work(const char* name, double work);
 
+// ------------------------------------------------------------------ host copies
+// Copies between pageable host arrays and the device through pinned staging
+// memory, the pageable side by several threads (csrc/fs_stage.cpp).  An object
+// that makes such copies holds a HostStage; the staging memory is shared by all of
+// them, at most kStages pieces, and given back when the last one goes.
+struct HostCopy {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+class HostStage {
+   public:
+    HostStage();
+    ~HostStage();
+    HostStage(const HostStage&) = delete;
+    HostStage& operator=(const HostStage&) = delete;
+    // Device to host on `st`; the host arrays are filled when it returns.
+    void to_host(const std::vector<HostCopy>& copies, cudaStream_t st);
+    // Host to device on `st`; the host arrays have been read when it returns, the
+    // device arrays are written in stream order.
+    void to_device(const std::vector<HostCopy>& copies, cudaStream_t st);
+};
+
 // ------------------------------------------------------------------ device buffers
 // Bumped by every device (re)allocation of a DevBuf; a captured CUDA graph
 // records it and is discarded when it changed, since the graph's kernels hold
