@@ -66,7 +66,9 @@ __global__ void k_cell_keys(CellPlan P, const double* __restrict__ x, int n, uin
 // both only grow along the sorted points, so (sub-chunk + cell) numbers the
 // partials without a scan.  Balanced whatever the points' distribution: a
 // thread's work does not depend on how many points a cell holds.  Also writes
-// each cell's first sorted point.
+// each cell's first sorted point.  kSorted: x (wrapped) and q are in order
+// themselves, skey and sidx are not read; a NaN at the end counts to cell 0.
+template <bool kSorted>
 __global__ void __launch_bounds__(256) k_cell_moments(CellPlan P, const uint32_t* __restrict__ skey,
                                                       const int* __restrict__ sidx, const double* __restrict__ x,
                                                       const double* __restrict__ q, int n, int* __restrict__ start,
@@ -76,13 +78,13 @@ __global__ void __launch_bounds__(256) k_cell_moments(CellPlan P, const uint32_t
     const int t = threadIdx.x, i = blockIdx.x * 256 + t;
     int key = P.M;  // beyond the last point
     if (i < n) {
-        key = (int)skey[i];
-        const int prev = i > 0 ? (int)skey[i - 1] : -1;
+        key = kSorted ? cell_of(x[i], P) : (int)skey[i];
+        const int prev = i > 0 ? (kSorted ? cell_of(x[i - 1], P) : (int)skey[i - 1]) : -1;
         for (int c = prev + 1; c <= key; ++c) start[c] = i;
         if (i == n - 1)
             for (int c = key + 1; c <= P.M; ++c) start[c] = n;
-        const int id = sidx[i];
-        const double w = cell_wrap(x[id], P.L), qi = q[id];
+        const int id = kSorted ? i : sidx[i];
+        const double w = kSorted ? x[id] : cell_wrap(x[id], P.L), qi = q[id];
         const double xi = fma(w, P.two_inv_h, -(double)(2 * key + 1));
         double a = qi, b = qi * xi;
         const double x2 = xi + xi;
@@ -208,6 +210,8 @@ struct CellSums {
     int Mc;
 };
 
+// kNear: with the near groups (else the one half a period away alone).
+template <bool kNear>
 __device__ __forceinline__ void cell_near(const CellSums& J, int g, CellSmem& S, int* __restrict__ err) {
     const int t = threadIdx.x, l = t & 15, k = (t >> 4) & 15, half = t >> 8;
     const int Mc = J.Mc;
@@ -245,7 +249,7 @@ __device__ __forceinline__ void cell_near(const CellSums& J, int g, CellSmem& S,
     const int i0 = half * 8;
     const double* T = J.tab + k * kP + l;
     // near offsets m = o - 32: source cell i - m, stored at i - m + 31
-    slide<8>(T, kNearOff, [&](int d) { return S.near_m[i0 + d + 63][k]; }, acc);
+    if (kNear) slide<8>(T, kNearOff, [&](int d) { return S.near_m[i0 + d + 63][k]; }, acc);
     // seam offsets m = o - 16: stored at i - m + 15
     slide<8>(T + (size_t)kNearOff * kPP, kSeamOff, [&](int d) { return S.seam_m[i0 + d + 31][k]; }, acc);
     __syncthreads();  // the shares take the moments' place
@@ -261,7 +265,8 @@ __device__ __forceinline__ void cell_near(const CellSums& J, int g, CellSmem& S,
     }
 }
 
-__device__ __forceinline__ void cell_far(const CellSums& J, int f, CellSmem& S) {
+__device__ __forceinline__ void cell_far(const CellSums& J, const double* __restrict__ far_tab,
+                                         double* __restrict__ locc, int f, CellSmem& S) {
     const int t = threadIdx.x, l = t & 15, k = (t >> 4) & 15, half = t >> 8;
     const int Mc = J.Mc, g0 = f * kFarGroups;
     // offsets in two halves of a multiple of 4 (the table is zero from Mc on)
@@ -269,7 +274,7 @@ __device__ __forceinline__ void cell_far(const CellSums& J, int f, CellSmem& S) 
     const int o0 = half * n;
     const double* __restrict__ W = J.momc + k;
     double acc[kFarGroups] = {0, 0, 0, 0};
-    slide<kFarGroups>(J.tab + (size_t)(kNearOff + kSeamOff + o0) * kPP + k * kP + l, n,
+    slide<kFarGroups>(far_tab + (size_t)o0 * kPP + k * kP + l, n,
                       [&](int d) {
                           int s = g0 - o0 + d;  // above -2 Mc - 8
                           s += s < 0 ? Mc : 0;
@@ -286,7 +291,7 @@ __device__ __forceinline__ void cell_far(const CellSums& J, int f, CellSmem& S) 
         double s = 0.0;
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk) s += S.red[kk][i][0][l] + S.red[kk][i][1][l];
-        J.locc[(size_t)(g0 + i) * kP + l] = s;
+        locc[(size_t)(g0 + i) * kP + l] = s;
     }
 }
 
@@ -296,8 +301,36 @@ __global__ void __launch_bounds__(kPairT) k_cell_pairs(CellSums J, int* __restri
     __shared__ __align__(128) CellSmem S;
     const int nf = (J.Mc + kFarGroups - 1) / kFarGroups;
     const int b = blockIdx.x;  // far items first: theirs is the longer chain of L2 reads
-    if (b < nf) cell_far(J, b, S);
-    else cell_near(J, b - nf, S, err);
+    if (b < nf) cell_far(J, J.tab + (size_t)(kNearOff + kSeamOff) * kPP, J.locc, b, S);
+    else cell_near<true>(J, b - nf, S, err);
+}
+
+// What a windowed sum leaves to the cells: for every group the other groups'
+// share without those of a window about itself, and again about the group before
+// it (targets of a block that runs over into the next group), and for every cell
+// the group half a period away.  15 us at 158 groups, beside 8.1 ms of pairs.
+__global__ void __launch_bounds__(kPairT) k_cell_rest(CellSums J, const double* __restrict__ rest_tab,
+                                                      int* __restrict__ err) {
+    __shared__ __align__(128) CellSmem S;
+    const int nf = (J.Mc + kFarGroups - 1) / kFarGroups, noff = (J.Mc + 7) / 8 * 8;
+    const int b = blockIdx.x;
+    if (b < 2 * nf) {
+        const int v = b >= nf;
+        cell_far(J, rest_tab + (size_t)v * noff * kPP, J.locc + (size_t)v * J.Mc * kP, b - v * nf, S);
+    } else {
+        cell_near<false>(J, b - 2 * nf, S, err);
+    }
+}
+
+// Group offsets with the window's left out: |m| <= kWinGroups, and then shifted by one.
+__global__ void __launch_bounds__(kPP) k_rest_table(CellPlan P, const double* __restrict__ tab,
+                                                    double* __restrict__ rest) {
+    const int noff = (P.Mc + 7) / 8 * 8, v = blockIdx.x / noff, m = blockIdx.x % noff;
+    int c = m - v;  // offset from the window's middle, about 0
+    if (c > P.Mc / 2) c -= P.Mc;
+    const bool out = c >= -kWinGroups && c <= kWinGroups;
+    const double t = tab[(size_t)(kNearOff + kSeamOff + m) * kPP + threadIdx.x];
+    rest[(size_t)blockIdx.x * kPP + threadIdx.x] = out ? 0.0 : t;
 }
 
 // E at the targets (in the caller's order: coalesced stage arrays; a cell's
@@ -431,7 +464,7 @@ void cell_field(const CellPlan& P, const CellBuffers& B, const double* d_t, int 
     k_cell_keys<<<nb, T, 0, st>>>(P, d_s, ns, B.kin, B.iin);
     size_t tb = B.sort_bytes;
     FS_CUDA(cub::DeviceRadixSort::SortPairs(B.sort_tmp, tb, B.kin, B.kout, B.iin, B.iout, ns, 0, key_bits(P.M), st));
-    k_cell_moments<<<nb, T, 0, st>>>(P, B.kout, B.iout, d_s, d_q, ns, B.start, B.part);
+    k_cell_moments<false><<<nb, T, 0, st>>>(P, B.kout, B.iout, d_s, d_q, ns, B.start, B.part);
     k_cell_gather<<<P.Mc, 1024, 0, st>>>(P, B.start, B.part, B.child, B.mom, B.momc);
     {
         ProfScope prof("k_cell_pairs", st, (double)nt * (double)ns);
@@ -440,6 +473,23 @@ void cell_field(const CellPlan& P, const CellBuffers& B, const double* d_t, int 
     }
     k_cell_eval<<<(nt + T - 1) / T, T, 0, st>>>(P, d_t, nt, B.loc, B.locc, S);
     FS_LAUNCHED(5);
+}
+
+size_t cell_rest_table_size(const CellPlan& P) { return 2 * (size_t)((P.Mc + 7) / 8 * 8) * kPP; }
+
+void cell_rest_table(const CellPlan& P, const double* tab, double* rest_tab, cudaStream_t st) {
+    k_rest_table<<<2 * ((P.Mc + 7) / 8 * 8), kPP, 0, st>>>(P, tab, rest_tab);
+    FS_LAUNCHED(1);
+}
+
+void cell_rest(const CellPlan& P, const CellBuffers& B, const double* rest_tab, const double* d_x, const double* d_q,
+               int ns, double* locc2, int* err, cudaStream_t st) {
+    const int T = 256, nb = (ns + T - 1) / T;
+    k_cell_moments<true><<<nb, T, 0, st>>>(P, nullptr, nullptr, d_x, d_q, ns, B.start, B.part);
+    k_cell_gather<<<P.Mc, 1024, 0, st>>>(P, B.start, B.part, B.child, B.mom, B.momc);
+    k_cell_rest<<<2 * cell_far_items(P.Mc) + P.Mc, kPairT, 0, st>>>(
+        CellSums{B.mom, B.momc, B.tab, B.loc, locc2, P.Mc}, rest_tab, err);
+    FS_LAUNCHED(3);
 }
 
 void set_cell_polls(long long polls) {

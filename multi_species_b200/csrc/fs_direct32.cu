@@ -34,6 +34,10 @@
 //    move global->shared by TMA bulk copies (cp.async.bulk, no multicast),
 //    double-buffered on mbarriers.
 //
+//  * Self-fields asked for pairwise, of many points (Direct32c::windowed), sum
+//    pairs within a window of cells about each target block and take the rest
+//    from cell expansions (csrc/fs_cells.cu).
+//
 // Work is split into (target block, source chunk) items, taken from an atomic
 // counter by a one-wave persistent grid in an order estimated on the device
 // (band-heavy items spread over the queue, light ones last); chunk partials are
@@ -43,9 +47,10 @@
 
 #include <cstdlib>
 #include <mutex>
+#include <vector>
 
 #include "fs_bulk.cuh"
-#include "fs_device.cuh"
+#include "fs_cells.cuh"
 
 namespace fsb {
 
@@ -106,6 +111,11 @@ __global__ void k_wrap_keys(const double* __restrict__ x, int n, double L, uint6
 __device__ __forceinline__ float4 source_record(double s, double q, double a1, double a2) {
     const float qh = (float)(0.5 * q);
     return make_float4((float)s, qh, (float)((double)qh * a1), (float)((double)qh * a2));
+}
+
+__global__ void k_sorted_x(const uint64_t* __restrict__ keys, int n, double* __restrict__ x) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) x[i] = key_to_x(keys[i]);
 }
 
 // Sorted sources -> tile-relative FP32 records {s, q/2, q/2 a1, q/2 a2}
@@ -271,15 +281,25 @@ constexpr double kCellLoad = 2e7;  // n L / epsilon from which sums go through c
 // `gk` counts the tiles this CTA has consumed (buffer = gk & 1, barrier phase
 // = (gk >> 1) & 1), so the barriers keep alternating across work items.
 // Returns false when a bounded wait gave up (flag set, CTA must stop).
-template <int kR>
+// kWin: the chunk is of the tiles of the block's window (Jb.win); of a tile at its
+// end only the sources inside are summed, one by one.
+template <int kR, bool kWin = false>
 __device__ __forceinline__ bool pair_block(const PairJob& Jb, int tb, int chunk, float4 (*buf)[kS],
                                            double2 (*buf64)[kS], uint64_t* bar,
                                            uint32_t& gk, int* __restrict__ err) {
     constexpr int kTB = kNT * kR;
     const int tid = threadIdx.x;
+    PairWindow W;
+    if (kWin) W = Jb.win[tb];
     const int t0 = chunk * Jb.tpc;
-    const int t1 = min(Jb.ntiles, t0 + Jb.tpc);
+    const int t1 = min(kWin ? W.nt : Jb.ntiles, t0 + Jb.tpc);
     if (t0 >= t1) return true;
+    const int ntiles = Jb.ntiles;
+    auto tile_at = [&](int k) {
+        if (!kWin) return k;
+        const int t = W.t0 + k;
+        return t >= ntiles ? t - ntiles : t;
+    };
     const float eps2 = Jb.eps2, a1 = Jb.a1, a2 = Jb.a2;
     const double L = Jb.L;
     const int ns = Jb.ns;
@@ -307,16 +327,18 @@ __device__ __forceinline__ bool pair_block(const PairJob& Jb, int tb, int chunk,
     if (tid == 0) {
         fence_proxy_async();
         mbar_expect_tx(&bar[gk & 1], kBytes + kBytes64);
-        bulk_load(buf[gk & 1], Jb.src + (size_t)t0 * kS, kBytes, &bar[gk & 1]);
-        if (kStage64) bulk_load(buf64[gk & 1], Jb.src64 + (size_t)t0 * kS, kBytes64, &bar[gk & 1]);
+        const int t = tile_at(t0);
+        bulk_load(buf[gk & 1], Jb.src + (size_t)t * kS, kBytes, &bar[gk & 1]);
+        if (kStage64) bulk_load(buf64[gk & 1], Jb.src64 + (size_t)t * kS, kBytes64, &bar[gk & 1]);
     }
-    for (int t = t0; t < t1; ++t, ++gk) {
-        const int b = gk & 1;
-        if (tid == 0 && t + 1 < t1) {
+    for (int kt = t0; kt < t1; ++kt, ++gk) {
+        const int b = gk & 1, t = tile_at(kt);
+        if (tid == 0 && kt + 1 < t1) {
+            const int tn = tile_at(kt + 1);
             fence_proxy_async();
             mbar_expect_tx(&bar[b ^ 1], kBytes + kBytes64);
-            bulk_load(buf[b ^ 1], Jb.src + (size_t)(t + 1) * kS, kBytes, &bar[b ^ 1]);
-            if (kStage64) bulk_load(buf64[b ^ 1], Jb.src64 + (size_t)(t + 1) * kS, kBytes64, &bar[b ^ 1]);
+            bulk_load(buf[b ^ 1], Jb.src + (size_t)tn * kS, kBytes, &bar[b ^ 1]);
+            if (kStage64) bulk_load(buf64[b ^ 1], Jb.src64 + (size_t)tn * kS, kBytes64, &bar[b ^ 1]);
         }
         const bool ok = mbar_wait_bounded(&bar[b], (gk >> 1) & 1, polls);
         if (!__syncthreads_and(ok)) {
@@ -327,15 +349,22 @@ __device__ __forceinline__ bool pair_block(const PairJob& Jb, int tb, int chunk,
                 // buf[b ^ 1].  Shared memory is released when the CTA exits,
                 // so let both land first (bounded waits).
                 (void)mbar_wait_bounded(&bar[b], (gk >> 1) & 1, kMbarPolls);
-                if (t + 1 < t1) (void)mbar_wait_bounded(&bar[b ^ 1], ((gk + 1) >> 1) & 1, kMbarPolls);
+                if (kt + 1 < t1) (void)mbar_wait_bounded(&bar[b ^ 1], ((gk + 1) >> 1) & 1, kMbarPolls);
             }
             return false;
         }
         const double base = Jb.tbase[t];
         const int jlo = t * kS;
         const int jend = min(jlo + kS, ns);  // real sources in this tile
+        // sources [ja, jb) of the tile; a window's ends cut its first and last tile
+        int ja = 0, jb = kS;
+        if (kWin && W.group >= 0) {
+            const int e = W.s1 + W.len - (W.s1 + W.len > ns && jend <= W.s1 ? ns : 0);  // end, in the tile's turn
+            ja = jlo < W.s1 && jend > W.s1 && kt == 0 ? W.s1 - jlo : 0;
+            jb = min(kS, max(e - jlo, 0));
+        }
         float tau[kR], tauh[kR], sg[kR], acc[kR];
-        bool careful = false, inband = true;
+        bool careful = kWin && (ja > 0 || jb < jend - jlo), inband = !careful;
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
             const double lo = tl[r] - base;
@@ -440,7 +469,7 @@ __device__ __forceinline__ bool pair_block(const PairJob& Jb, int tb, int chunk,
             float cmp[kR];
 #pragma unroll
             for (int r = 0; r < kR; ++r) cmp[r] = 0.f;
-            for (int j = 0; j < kS; ++j) {
+            for (int j = kWin ? ja : 0; j < (kWin ? jb : kS); ++j) {
                 const float4 e = tile[j];
                 const int idx = jlo + j;
 #pragma unroll
@@ -543,7 +572,7 @@ constexpr int kMinBlocks8 = FS_MIN_BLOCKS8;
 // items from an atomic counter, in the order `order` gives (band-heavy items
 // spread over the queue, light ones last) or in chunk-major order when it is
 // null.
-template <int kR>
+template <int kR, bool kWin = false>
 __global__ void __launch_bounds__(kNT, (kR >= 8 ? kMinBlocks8 : 8) * 128 / kNT) k_pairs32_persistent(PairJob job, int tblocks, int nitems,
                                                             const int* __restrict__ order,
                                                             int* __restrict__ counter, int* __restrict__ err) {
@@ -562,7 +591,7 @@ __global__ void __launch_bounds__(kNT, (kR >= 8 ? kMinBlocks8 : 8) * 128 / kNT) 
         const int item = s_item;
         __syncthreads();
         if (item >= nitems) break;
-        if (!pair_block<kR>(job, item % tblocks, item / tblocks, buf, buf64, bar, gk, err)) return;
+        if (!pair_block<kR, kWin>(job, item % tblocks, item / tblocks, buf, buf64, bar, gk, err)) return;
     }
 }
 
@@ -592,14 +621,18 @@ __device__ __forceinline__ double target_x(const TargetInfo& T, double L) { retu
 // Sort key of an item: its estimated cost, with kHeavy set when it has tiles
 // within the band; counts heavy items into *nheavy.
 __device__ int item_key(const PairJob& J, int tb, int c, int ttb, int* __restrict__ nheavy) {
-    const int t0 = c * J.tpc, t1 = min(J.ntiles, t0 + J.tpc);
+    const bool win = J.win && J.win[tb].group >= 0;
+    const int first_tile = win ? J.win[tb].t0 : 0;
+    const int t0 = c * J.tpc, t1 = min(win ? J.win[tb].nt : J.ntiles, t0 + J.tpc);
     if (t0 >= t1 || J.nt <= 0) return 0;
     // the block's real targets, sorted by x: the first and the last bound it
     const int first = min(tb * ttb, J.nt - 1), last = min(tb * ttb + ttb, J.nt) - 1;
     const double xa = target_x(J.info[first], J.L), xb = target_x(J.info[last], J.L);
     const double band = kBand * sqrt(J.eps2d);
     int near = 0;
-    for (int t = t0; t < t1; ++t) {
+    for (int k = t0; k < t1; ++k) {
+        int t = first_tile + k;
+        t -= t >= J.ntiles ? J.ntiles : 0;
         const double ya = J.tbase[t];
         const double yb = (t + 1 < J.ntiles) ? J.tbase[t + 1] : J.L;
         double gap = 1e300;
@@ -772,6 +805,86 @@ __global__ void k_finalize32(const double* __restrict__ partial, int nchunks, in
         const double B = T.tlo * Q - qxsum[0] + L * (Q - PJ);
         E += form_ffar ? far_sign_sum(T, pq, ns) : T.ffar;
         E -= cbg * B;
+    }
+    apply_stage(S, tperm[i], E);
+}
+
+// ---------------------------------------------------------------- windowed sums
+// The window of every target block: the groups of cells within kWinGroups of the
+// block's first target's, as a range of sorted sources (a block over more than
+// two groups takes all sources).
+__global__ void k_windows(CellPlan P, const uint64_t* __restrict__ tkeys, int nt, int ttb, int nblocks,
+                          const int* __restrict__ start, int ns, int ntiles, PairWindow* __restrict__ win) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nblocks) return;
+    PairWindow W{0, ns, 0, ntiles, -1};
+    const int first = b * ttb, last = min(first + ttb, nt) - 1;
+    // (a NaN among the positions is the last of them, and reaches every sum)
+    if (first <= last && !isnan(key_to_x(tkeys[nt - 1]))) {
+        const int ga = cell_of(key_to_x(tkeys[first]), P) / kCellGroup, gb = cell_of(key_to_x(tkeys[last]), P) / kCellGroup;
+        if (gb - ga <= 1) {
+            int lo = ga - kWinGroups, hi = ga + kWinGroups + 1;
+            int turn_lo = 0, turn_hi = 0;
+            if (lo < 0) {
+                lo += P.Mc;
+                turn_lo = -ns;
+            }
+            if (hi > P.Mc) {
+                hi -= P.Mc;
+                turn_hi = ns;
+            }
+            const int a = start[lo * kCellGroup] + turn_lo, e = start[hi * kCellGroup] + turn_hi;
+            W.s1 = a < 0 ? a + ns : a;
+            W.len = e - a;
+            W.group = ga;
+            if (W.s1 == ns) W.s1 = 0;  // the groups below the wrap hold no sources
+            if (W.len > 0) {
+                const int end = W.s1 + W.len - 1;  // last source, in the window's turn
+                W.t0 = W.s1 / kS;
+                W.nt = (end < ns ? end / kS : ntiles + (end - ns) / kS) - W.t0 + 1;
+                if (W.nt > ntiles) W = PairWindow{0, ns, 0, ntiles, -1};  // the window meets itself in one tile
+            } else {
+                W.t0 = W.nt = 0;
+            }
+        }
+    }
+    win[b] = W;
+}
+
+// E of windowed sums: the chunk partials of the block's window, its exact sign sum
+// and background from prefix sums, and what the cells sum outside it.
+__global__ void k_finalize_win(PairJob J, int ttb, const double* __restrict__ x, const double* __restrict__ pq, const double* __restrict__ pqx,
+                               double cbg, const int* __restrict__ tperm, CellPlan P, const double* __restrict__ loc,
+                               const double* __restrict__ locc2, Stage S) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= J.nt) return;
+    const PairWindow W = J.win[i / ttb];
+    const int nch = (W.nt + J.tpc - 1) / J.tpc, ns = J.ns;
+    double E = 0.0;
+    for (int c = 0; c < nch; ++c) E += J.partial[(size_t)c * J.nt_pad + i];
+    const TargetInfo T = J.info[i];
+    const double L = J.L;
+    int w1 = T.J, w2 = T.J + ns;
+    if (W.group >= 0) {
+        w1 = W.s1 >= T.J ? W.s1 : W.s1 + ns;
+        w2 = min(w1 + W.len, T.J + ns);
+    }
+    auto px = [&](int u) {  // sum of q X over unrolled [0, u)
+        const int r = u >= ns ? u - ns : u;
+        double v = r ? pqx[r - 1] : 0.0;
+        if (u >= ns) v += pqx[ns - 1] + L * (r ? pq[r - 1] : 0.0);
+        return v;
+    };
+    const double p1 = unrolled_prefix(pq, ns, w1), p2 = unrolled_prefix(pq, ns, w2);
+    E += 0.5 * ((unrolled_prefix(pq, ns, T.U1) - p1) - (p2 - unrolled_prefix(pq, ns, T.U2)));
+    E -= cbg * ((T.tlo + L) * (p2 - p1) - (px(w2) - px(w1)));
+    if (W.group >= 0) {
+        const double xt = x[i];
+        const int c = cell_of(xt, P), g = c / kCellGroup;
+        const double xi = fma(xt, P.two_inv_h, -(double)(2 * c + 1));
+        const double xg = fma(xt, P.two_inv_h, -(double)((2 * g + 1) * kCellGroup)) * (1.0 / kCellGroup);
+        const double* far = locc2 + (size_t)(g == W.group ? 0 : P.Mc) * kCellTerms;
+        E += cheb_sum(loc + (size_t)c * kCellTerms, xi) + cheb_sum(far + (size_t)g * kCellTerms, xg);
     }
     apply_stage(S, tperm[i], E);
 }
@@ -1082,7 +1195,7 @@ void small_field(const SmallBuffers& B, double L, double eps, const double* d_t,
                                                                 e2 * e2 / 8, B.src, B.src64, B.tbase, B.pq, B.qxsum,
                                                                 B.tkout, nt, nt_pad, L, kBand * eps, B.info);
     const PairJob job{B.src, B.src64, B.tbase, B.info, B.partial, ns, ntiles, 1, nt_pad, L, (float)e2,
-                      (float)(e2 / 2), (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, nt};
+                      (float)(e2 / 2), (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, nt, nullptr};
     {
         ProfScope prof("k_pairs32", st, (double)nt * (double)ns);
         const dim3 grid((nt + group - 1) / group, ntiles);
@@ -1138,6 +1251,10 @@ class Direct32c final : public FieldEngine {
             const SmallBuffers B{kout_.p, same ? kout_.p : tkout_.p, iout_.p, same ? iout_.p : tiout_.p, src_.p,
                                  src64_.p, tbase_.p, pq_.p, qxsum_.p, partial_.p, info_.p};
             small_field(B, L_, eps_, d_t, nt, d_s, d_q, ns, nt_pad, 32 * R_, stage, err_.p, false, st);
+            return;
+        }
+        if (form == PairForm::pairwise && d_t == d_s && nt == ns && windowed(ns)) {
+            eval_windowed(d_s, d_q, ns, stage, st);
             return;
         }
         // a standalone launch: one persistent wave over about 32 items per CTA
@@ -1218,7 +1335,7 @@ class Direct32c final : public FieldEngine {
         FS_LAUNCHED(1);
         last_nt_ = nt;
         *job = PairJob{src_.p, src64_.p, tbase_.p, info_.p, partial_.p, ns, ntiles, tpc, nt_pad, L_, (float)e2,
-                       (float)(e2 / 2), (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, nt};
+                       (float)(e2 / 2), (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, nt, nullptr};
         return true;
     }
 
@@ -1232,6 +1349,59 @@ class Direct32c final : public FieldEngine {
     }
 
     int* error_flag() override { return err_.p; }
+
+    // A self-field whose pairs beyond 60 to 70 epsilon go through cells, the nearer
+    // ones pair by pair as always: the far terms fall as eps^2 / d^2 and so does
+    // their rounding, 1e-11 of E for all that lies beyond the window (measured
+    // against all pairs: 5e-12 of E at 66,049 points, 2e-12 at 525,825; with
+    // windows of 40 epsilon 9e-12 and 3e-12, of 100 epsilon 3e-12 and 1e-12).  At
+    // 525,825 points of the two-stream box the windows hold 8% of the pairs and E
+    // takes 8.5 ms in place of 42.6; 11.5 ms with windows of 100 epsilon, 7.2 with
+    // 40.  Below 50,000 points it is no faster (33,153: 0.5 ms either way), and in
+    // boxes below 640 epsilon the windows hold a fifth of the pairs and more.
+    bool windowed(int n) const { return cells_ && R_ == 8 && n >= 50000 && plan_.Mc >= 64; }
+    void eval_windowed(const double* d_x, const double* d_q, int n, const Stage& stage, cudaStream_t st) {
+        const int ntiles = (n + kS - 1) / kS, nt_pad = (n + kTBPad - 1) / kTBPad * kTBPad;
+        const int ttb = kNT * R_, tblocks = nt_pad / ttb, tpc = (ntiles + kMaxChunks - 1) / kMaxChunks;
+        const int nchunks = (ntiles + tpc - 1) / tpc, nitems = tblocks * nchunks;
+        if (!grid_) grid_ = persistent_grid(R_);
+        PairJob job;
+        if (!prepare(d_x, n, d_x, d_q, n, stage, st, tpc, &job)) return;
+        // the cells' part, on the sorted sources
+        reserve_cells(n);
+        const size_t rest = cell_rest_table_size(plan_);
+        if (!rest_.p) {
+            // once, before any (non-blocking) stream reads it
+            rest_.ensure(rest);
+            cell_rest_table(plan_, buf_.tab, rest_.p, nullptr);
+            FS_CUDA(cudaStreamSynchronize(nullptr));
+        }
+        locc2_.ensure(2 * (size_t)plan_.Mc * kCellTerms);
+        xs_.ensure(n);
+        pqx_.ensure(n);
+        win_.ensure(tblocks);
+        const int T = 256;
+        k_sorted_x<<<(n + T - 1) / T, T, 0, st>>>(kout_.p, n, xs_.p);
+        scan_f64_inclusive(qx_.p, pqx_.p, n, scan_.p, st);
+        cell_rest(plan_, buf_, rest_.p, xs_.p, qs_.p, n, locc2_.p, err_.p, st);
+        k_windows<<<(tblocks + T - 1) / T, T, 0, st>>>(plan_, kout_.p, n, ttb, tblocks, start_.p, n, ntiles, win_.p);
+        FS_LAUNCHED(2);
+        job.win = win_.p;
+        const int* order = item_order(nitems, tblocks, job, st);
+        {
+            const double work = profiling_enabled() ? window_pairs(n, ttb, st) : 0.0;
+            ProfScope prof("k_pairs32", st, work);
+            FS_CUDA(cudaMemsetAsync(counter_.p, 0, sizeof(int), st));
+            k_pairs32_persistent<8, true><<<std::min(grid_, nitems), kNT, 0, st>>>(job, tblocks, nitems, order,
+                                                                                  counter_.p, err_.p);
+            FS_LAUNCHED(1);
+        }
+        fin_.pending = false;
+        k_finalize_win<<<(n + T - 1) / T, T, 0, st>>>(job, ttb, xs_.p, pq_.p, pqx_.p, cbg_, iout_.p, plan_, buf_.loc, locc2_.p,
+                                                      stage);
+        FS_LAUNCHED(1);
+    }
+
     // The two forms of the sum agree to the pairwise one's FP32 error: 2e-10 of E
     // at L = 250 epsilon whatever n, falling as epsilon / L, and more for few
     // points (1e-9 at 600).  Cells take over where that leaves E within a few
@@ -1259,6 +1429,16 @@ class Direct32c final : public FieldEngine {
     }
 
    private:
+    // Pairs inside the windows (while profiling: waits for the stream).
+    double window_pairs(int nt, int ttb, cudaStream_t st) {
+        std::vector<PairWindow> w((nt + ttb - 1) / ttb);
+        FS_CUDA(cudaMemcpyAsync(w.data(), win_.p, w.size() * sizeof(PairWindow), cudaMemcpyDeviceToHost, st));
+        FS_CUDA(cudaStreamSynchronize(st));
+        double pairs = 0.0;
+        for (size_t b = 0; b < w.size(); ++b) pairs += (double)std::min(ttb, nt - (int)b * ttb) * w[b].len;
+        return pairs;
+    }
+
     // The persistent launch's items in the order of order_items (heavy items
     // spread over the queue, light ones last).
     const int* item_order(int nitems, int tblocks, const PairJob& job, cudaStream_t st) {
@@ -1366,6 +1546,9 @@ class Direct32c final : public FieldEngine {
     DevBuf<uint32_t> ckeys_;
     DevBuf<double> part_, coef_, tab_;
     DevBuf<int> start_;
+    // windowed sums
+    DevBuf<double> rest_, locc2_, xs_, pqx_;
+    DevBuf<PairWindow> win_;
 };
 
 }  // namespace
@@ -1583,7 +1766,7 @@ void direct32c_noalloc(double L, double eps, double* d_es, const double* d_x, co
     sum_f64(qx, n, reinterpret_cast<double*>(cub_tmp), qxsum, st);
     k_target_info<<<(nt_pad + T - 1) / T, T, 0, st>>>(kout, n, nt_pad, kout, n, L, kBand * eps, pq, info);
     const PairJob job{src, src64, tbase, info, partial, n, ntiles, tpc, nt_pad, L, (float)e2, (float)(e2 / 2),
-                      (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, n};
+                      (float)(e2 * e2 / 8), (float)(0.75 * e2), e2, n, nullptr};
     launch_pairs(R, dim3(tblocks, nchunks), st, job, err);
     const double cbg = 1 / std::sqrt(L * L + 4 * eps * eps);
     k_finalize32<<<(n + T - 1) / T, T, 0, st>>>(partial, nchunks, nt_pad, n, info, pq, qxsum, n, L, cbg, iout, false, S);

@@ -226,6 +226,14 @@ struct PairJob {
     float e2f;           // far pairs: 3 eps^2 / 4
     double eps2d;        // band pairs (FP64): eps^2
     int nt;              // targets: the first nt of the nt_pad entries of info are real
+    // Windowed sums: per target block the sources that are summed here, a cyclic
+    // range of the sorted ones (null: all).
+    const struct PairWindow* win;
+};
+struct PairWindow {
+    int s1, len;      // sorted sources s1, s1 + 1, ... (modulo ns)
+    int t0, nt;       // tiles that hold them: t0, t0 + 1, ... (modulo ntiles)
+    int group;        // their middle group of cells, or -1: all sources
 };
 
 // Cell expansions of the periodic direct sum (csrc/fs_cells.cu).
@@ -264,6 +272,16 @@ void cell_offset_table(const CellPlan& P, double* tab, cudaStream_t st);
 // that gave up.
 void cell_field(const CellPlan& P, const CellBuffers& B, const double* d_t, int nt, const double* d_s,
                 const double* d_q, int ns, const Stage& S, int* err, cudaStream_t st);
+// The part of a windowed sum that the pairs leave out (csrc/fs_cells.cu,
+// k_cell_rest): tables with the window's groups left out, and the evaluation's
+// coefficients.  x (wrapped), q: the sorted sources.
+constexpr int kWinGroups = 6;   // groups to either side of a window's middle
+size_t cell_rest_table_size(const CellPlan& P);
+void cell_rest_table(const CellPlan& P, const double* tab, double* rest_tab, cudaStream_t st);
+// locc holds 2 Mc * kCellTerms: groups seen from a window about themselves, then
+// about the group before.
+void cell_rest(const CellPlan& P, const CellBuffers& B, const double* rest_tab, const double* d_x, const double* d_q,
+               int ns, double* locc2, int* err, cudaStream_t st);
 void set_cell_polls(long long polls);
 
 // How an evaluation's pairs are summed where an engine has several ways: as it

@@ -83,3 +83,26 @@ def test_imported_field_is_the_next_steps_first():
     sa, sb = a.state(), b.state()
     for k in ("xs", "ps"):
         assert np.linalg.norm(sa[k] - sb[k]) <= 1e-8 * np.linalg.norm(sb[k]), k
+
+
+@pytest.mark.parametrize("ratio,kind", [
+    (600.0, "uniform"), (1570.8, "uniform"), (1570.8, "cell"), (1570.8, "cluster"), (1570.8, "lattice"),
+    (5119.0, "uniform"), (640.0, "uniform"), (640.0, "cluster"), (2500.0, "ends")])
+def test_exported_field_of_a_large_session(ratio, kind):
+    """E handed out of a session of 66,049 points (pairs within a window of cells,
+    the rest through cells; at 600 epsilon, and where a block of targets spans
+    more than two groups, all pairs): the pairwise kernel's 1e-9 of the band
+    charge, as above."""
+    rng = np.random.default_rng(int(ratio))
+    d = decks.two_stream(h=7, ph=0, remesh_period=100)
+    L = d["xmax"]
+    d.update(greens_epsilon=L / ratio, dt=1e-3)
+    s = M.Simulation(d, "direct32c")
+    n = s.n
+    x = L * (1 - rng.beta(0.1, 0.1, n)) if kind == "ends" else _points(kind, n, L, rng)
+    s.import_xp(xs=x, ps=np.zeros(n))
+    s.step(1)
+    st = s.state()
+    t = np.argsort(np.mod(st["xs"], L))[np.unique(np.r_[0, n - 1, rng.integers(0, n, 300)])]
+    ref = O.direct_sum(L, L / ratio, st["xs"][t], st["xs"], st["q_ws"])
+    assert np.max(np.abs(st["es"][t] - ref)) <= 2e-9 * np.sum(np.abs(st["q_ws"]))
