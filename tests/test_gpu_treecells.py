@@ -53,3 +53,40 @@ def test_fp32c_takes_the_same_sums():
     e32 = M.E_MQ_Treecode_B200(L, 0.05, 0.7, 8, 500, precision="fp32c").evaluate(x, x, q)
     e64 = M.E_MQ_Treecode_B200(L, 0.05, 0.7, 8, 500, precision="fp64").evaluate(x, x, q)
     assert np.max(np.abs(e32 - e64)) < 1e-12 * np.sum(np.abs(q))
+
+
+@pytest.mark.parametrize("n,kind,precision", [
+    (1, "spread", "fp64"), (2, "crowd", "fp32c"), (3000, "pairs", "fp64"), (20000, "crowd", "fp64"),
+    (20000, "crowd", "fp32c"), (60000, "crowds", "fp64"), (60000, "crowds", "fp32c"),
+    (1 << 18, "spread", "fp64"), ((1 << 18) + 1, "crowd", "fp64"), (400_000, "crowds", "fp32c")])
+def test_the_points_order_does_not_matter(n, kind, precision):
+    """Points with distinct positions are summed in the order of x, however close
+    together they are and however they come: the same bits in every order."""
+    rng = np.random.default_rng(n)
+    L = 4 * np.pi
+    if kind == "spread":
+        x = rng.uniform(-L, L, n)
+    elif kind == "pairs":     # neighbours 1e-13 apart
+        c = rng.uniform(0, L, n // 2)
+        x = np.r_[c, c + 1e-13]
+    elif kind == "crowd":     # 1,500 within 1e-10
+        x = rng.uniform(-L, L, n)
+        m = min(n, 1500)
+        x[:m] = 1.7 + 1e-10 * np.arange(m) / m
+    else:                     # groups of 2 .. 70 within 1e-11
+        x, k = np.empty(0), 2
+        while len(x) < n:
+            x = np.r_[x, rng.uniform(-0.9 * L, 0.9 * L) + 1e-11 * np.arange(k) / k]
+            if len(x) > 5000:
+                x = np.r_[x, rng.uniform(-L, L, n)]
+            k = 2 + (k + 31) % 69
+        x = x[:n]
+    x = np.unique(x)
+    q = rng.normal(size=len(x)) / n
+    eng = M.E_MQ_Treecode_B200(L, 0.05, 0.7, 8, 2000, precision=precision)
+    e = eng.evaluate(x, x, q)
+    for order in (rng.permutation(len(x)), np.arange(len(x))[::-1]):
+        assert np.array_equal(eng.evaluate(x[order], x[order], q[order]), e[order])
+    if len(x) <= 60000:
+        ref = O.treecode(L, 0.05, 0.7, 8, 2000, x, q)
+        assert np.max(np.abs(e - ref)) < (2e-12 if precision == "fp64" else 1e-8) * np.sum(np.abs(q))
