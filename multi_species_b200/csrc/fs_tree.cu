@@ -262,15 +262,41 @@ __device__ __forceinline__ void level_splits(const TNode* __restrict__ nodes, co
     }
 }
 
-// One CTA, level by level: all of a level's splits first (chains of dependent
-// loads, so as many lanes per node as there are to spare), then its children.
+// The splits of the first levels, by a node's place in the full binary tree (the
+// root 1, node h's children 2 h and 2 h + 1): the bisection does not depend on the
+// points, so every place of these levels finds its split at once, a thread each,
+// in place of a search per level one after another.
+constexpr int kHeapLevels = 14;
+inline int heap_levels(int n, int N0) {
+    int d = 1;
+    while (d < kHeapLevels && ((long long)N0 << (d - 2 > 0 ? d - 2 : 0)) < n) ++d;
+    return d;
+}
+__global__ void k_heap_splits(const double* __restrict__ sx, int n, int levels, int* __restrict__ heap) {
+    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h < 1 || h >= 1 << levels) return;
+    double x0 = sx[0] - 0.1234, x1 = sx[n - 1] + 0.001;
+    for (int b = 30 - __clz(h); b >= 0; --b) {
+        const double mid = 0.5 * (x0 + x1);
+        if (h >> b & 1) x0 = mid;
+        else x1 = mid;
+    }
+    heap[h] = upper_bound(sx, 0, n, 0.5 * (x0 + x1));
+}
+
+// One CTA, level by level: a level's splits (from the heap's levels, below them
+// all of a level's searches first, chains of dependent loads with as many lanes
+// per node as there are to spare), then its children.  Until a node of the heap's
+// levels is split, split[] holds its place there.
 // meta: [0] nodes, [1] leaves, [2] error code, [3] depth.  arrived[] is cleared
-// for the upward pass.  6.3 million points (13 levels): 204 -> 147 us,
-// 395,523 (9 levels): 88 -> 49 us, against a binary search per thread and level.
+// for the upward pass.  6.3 million points (13 levels): 62 us and 14 for
+// k_heap_splits, against 147 with every level's searches by lane groups and 204 by
+// a thread each; 395,523 (9 levels): 19 and 12, against 49 and 88.
 __global__ void __launch_bounds__(1024) k_build_tree(const double* __restrict__ sx, int n, int N0, int cap_nodes,
                                                      int cap_leaves, TNode* __restrict__ nodes,
                                                      int* __restrict__ leaves, int* __restrict__ split,
-                                                     int* __restrict__ arrived, int* __restrict__ meta) {
+                                                     int* __restrict__ arrived, const int* __restrict__ heap,
+                                                     int levels, int* __restrict__ meta) {
     __shared__ int s_begin, s_end, s_next, s_nleaf, s_err;
     __shared__ int s_child[32], s_leaf[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -285,6 +311,7 @@ __global__ void __launch_bounds__(1024) k_build_tree(const double* __restrict__ 
         r.parent = -1;
         r.level = 0;
         nodes[0] = r;
+        split[0] = 1;
         s_begin = 0;
         s_end = 1;
         s_next = 1;
@@ -299,19 +326,26 @@ __global__ void __launch_bounds__(1024) k_build_tree(const double* __restrict__ 
             break;
         }
         const int begin = s_begin, end = s_end, count = end - begin;
-        if (count <= 32) level_splits<32>(nodes, sx, N0, begin, end, split);
-        else if (count <= 128) level_splits<8>(nodes, sx, N0, begin, end, split);
-        else level_splits<1>(nodes, sx, N0, begin, end, split);
-        __syncthreads();
+        const bool known = level < levels;
+        if (!known) {
+            if (count <= 32) level_splits<32>(nodes, sx, N0, begin, end, split);
+            else if (count <= 128) level_splits<8>(nodes, sx, N0, begin, end, split);
+            else level_splits<1>(nodes, sx, N0, begin, end, split);
+            __syncthreads();
+        }
         for (int base = begin; base < end; base += 1024) {
             const int i = base + tid;
-            int nchild = 0, isleaf = 0, k = 0;
+            int nchild = 0, isleaf = 0, k = 0, place = 0;
             TNode nd;
             if (i < end) {
                 nd = nodes[i];
                 const int cnt = nd.m1 - nd.m0 + 1;
                 if (cnt >= N0) {
                     k = split[i];
+                    if (known) {
+                        place = k;
+                        k = min(max(heap[place], nd.m0), nd.m1 + 1);
+                    }
                     nchild = (k > nd.m0) + (k <= nd.m1);
                 } else {
                     isleaf = 1;
@@ -366,6 +400,7 @@ __global__ void __launch_bounds__(1024) k_build_tree(const double* __restrict__ 
                         ch.level = level + 1;
                         nodes[c] = ch;
                         arrived[c] = 0;
+                        split[c] = 2 * place;
                         c0 = c++;
                     }
                     if (k <= nd.m1 && c < cap_nodes) {
@@ -380,6 +415,7 @@ __global__ void __launch_bounds__(1024) k_build_tree(const double* __restrict__ 
                         ch.level = level + 1;
                         nodes[c] = ch;
                         arrived[c] = 0;
+                        split[c] = 2 * place + 1;
                         if (c0 < 0) c0 = c;
                         else c1 = c;
                         ++c;
@@ -1305,9 +1341,11 @@ class Treecode final : public FieldEngine {
         k_tree_runs<<<sm_count(), 1024, 0, st>>>(kout, runs_.p, nruns_.p, d_q, n, sx_.p, lam_.p, iin_.p, efar_.p,
                                                  iout_.p);
         const int* sidx = iin_.p;
-        FS_LAUNCHED(1);
+        FS_LAUNCHED(2);
+        const int levels = heap_levels(n, N0_);
+        k_heap_splits<<<((1 << levels) + 63) / 64, 64, 0, st>>>(sx_.p, n, levels, heap_.p);
         k_build_tree<<<1, 1024, 0, st>>>(sx_.p, n, N0_, cap_nodes, cap_leaves, nodes_.p, leaves_.p, split_.p,
-                                         arrived_.p, meta_.p);
+                                         arrived_.p, heap_.p, levels, meta_.p);
         k_mark_leaves<<<cap_leaves, 256, 0, st>>>(nodes_.p, leaves_.p, meta_.p, leaf_of_.p);
         k_lists<<<(cap_leaves + 3) / 4, 128, 0, st>>>(nodes_.p, leaves_.p, meta_.p, L_, std::sqrt(mac_ * mac_),
                                                           far_.p, far_n_.p, near_.p, near_n_.p, err_.p);
@@ -1397,6 +1435,7 @@ class Treecode final : public FieldEngine {
         near_.ensure((size_t)cap_leaves * kNearCap);
         near_n_.ensure(cap_leaves);
         split_.ensure(cap_nodes);
+        heap_.ensure((size_t)1 << kHeapLevels);
         arrived_.ensure(cap_nodes);
         mom_.ensure((size_t)cap_nodes * (kMaxDegree + 1));
         if (!err_.p) {
@@ -1416,7 +1455,7 @@ class Treecode final : public FieldEngine {
     double norm_ = 1, cbg_ = 0;
     DevBuf<uint32_t> keys_;
     DevBuf<double2> vq_;
-    DevBuf<int> runs_, nruns_, iin_, iout_, leaf_of_, leaves_, meta_, far_, far_n_, near_, near_n_, split_, arrived_, err_;
+    DevBuf<int> runs_, nruns_, iin_, iout_, leaf_of_, leaves_, meta_, far_, far_n_, near_, near_n_, split_, heap_, arrived_, err_;
     DevBuf<double> npart_, sx_, lam_, efar_, mom_, consts_, pl_, plx_, lx_, work_, scan_;
     int cap_leaves_ = 0;
     DevBuf<TNode> nodes_;
