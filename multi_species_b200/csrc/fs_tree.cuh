@@ -30,6 +30,11 @@ struct TreeView {
     int n, P, cap_leaves;
 };
 
+// A near leaf's slots (csrc/fs_treecells.cu).
+struct NearSlots {
+    int slot, n, c0;  // first slot, slots, first cell
+};
+
 // Near and far sums of every point through cells (csrc/fs_treecells.cu).
 class TreeCells {
    public:
@@ -41,8 +46,10 @@ class TreeCells {
 
    private:
     CellPlan plan_;
-    DevBuf<double> tab_, mom_, loc_;
-    DevBuf<int> leaf_c0_, leaf_slot_, slot_leaf_, chunk_leaf_, chunk_c_, count_;
+    DevBuf<double> tab_, mom_, loc_, part_;
+    DevBuf<NearSlots> near_;
+    DevBuf<int2> leaf_steps_, extra_;
+    DevBuf<int> leaf_chunk_, arrived_, leaf_c0_, leaf_slot_, slot_leaf_, chunk_leaf_, chunk_c_, count_;
 };
 
 }  // namespace fsb

@@ -90,3 +90,15 @@ def test_the_points_order_does_not_matter(n, kind, precision):
     if len(x) <= 60000:
         ref = O.treecode(L, 0.05, 0.7, 8, 2000, x, q)
         assert np.max(np.abs(e - ref)) < (2e-12 if precision == "fp64" else 1e-8) * np.sum(np.abs(q))
+
+
+@pytest.mark.parametrize("where", ["position", "charge"])
+@pytest.mark.parametrize("n", [1500, 1900])
+def test_nan_reaches_every_target(n, where):
+    """One leaf (n < 2000) through cells, its points in the upper half of the box."""
+    L = 4 * np.pi
+    x = np.linspace(0.5 * L, 0.9 * L, n)
+    q = np.full(n, -L / n)
+    (x if where == "position" else q)[n // 3] = np.nan
+    e = M.E_MQ_Treecode_B200(L, 0.2, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
+    assert np.all(np.isnan(e))
