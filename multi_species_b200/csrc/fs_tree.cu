@@ -1359,7 +1359,7 @@ class Treecode final : public FieldEngine {
         if (through_cells(n)) {
             const TreeView T{nodes_.p, leaves_.p, meta_.p, leaf_of_.p, far_.p, far_n_.p, near_.p, near_n_.p,
                              mom_.p, consts_.p, sx_.p, lam_.p, sidx, n, P_, cap_leaves};
-            ProfScope prof(fp32_ ? "k_near32" : "k_far_near64", st, last_pairs);
+            ProfScope prof("k_tree_cells", st, last_pairs);
             cells_.eval(T, N0_, norm_, stage, st);
             FS_LAUNCHED(7);
         } else if (!fp32_) {

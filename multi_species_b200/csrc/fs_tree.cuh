@@ -46,7 +46,7 @@ class TreeCells {
 
    private:
     CellPlan plan_;
-    DevBuf<double> tab_, mom_, loc_, part_;
+    DevBuf<double> tab_, mom_, loc_, part_, e_;
     DevBuf<NearSlots> near_;
     DevBuf<int2> leaf_steps_, extra_;
     DevBuf<int> leaf_chunk_, arrived_, leaf_c0_, leaf_slot_, slot_leaf_, chunk_leaf_, chunk_c_, count_;

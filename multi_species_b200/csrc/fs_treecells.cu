@@ -429,6 +429,16 @@ __global__ void __launch_bounds__(256) k_slot_eval(CellPlan P, TreeView T, const
     apply_stage(S, T.sidx[j], count[3] ? nan("") : E);
 }
 
+// The stage epilogue of fields formed in another order: a point's stage arrays are
+// six to eight scattered sectors from k_slot_eval, which at 6.3 million points (twice
+// the L2) takes 314 us on average over a step's stages (482 the last); E alone
+// scattered 75 and this 62 to 88.
+__global__ void __launch_bounds__(256) k_apply_stage(const double* __restrict__ E, int n, Stage S) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) apply_stage(S, i, E[i]);
+}
+constexpr int kApart = 1 << 20;  // points from which the stage arrays leave the L2
+
 }  // namespace
 
 bool TreeCells::init(double L, double eps) {
@@ -482,7 +492,18 @@ void TreeCells::eval(const TreeView& T, int max_source, double norm, const Stage
                       arrived_.p, count_.p, part_.p};
     if (wide) k_chunk_sums<16><<<cap_chunks, kPP, 0, st>>>(plan_, T, X, tab_.p, mom_.p, loc_.p);
     else k_chunk_sums<4><<<cap_chunks, kPP, 0, st>>>(plan_, T, X, tab_.p, mom_.p, loc_.p);
-    k_slot_eval<<<(T.n + 255) / 256, 256, 0, st>>>(plan_, T, leaf_c0_.p, leaf_slot_.p, count_.p, loc_.p, norm, S);
+    const bool apart = S.kind != STAGE_STORE && T.n >= kApart;
+    Stage field;
+    if (apart) {
+        e_.ensure(T.n);
+        field.out = e_.p;
+    }
+    k_slot_eval<<<(T.n + 255) / 256, 256, 0, st>>>(plan_, T, leaf_c0_.p, leaf_slot_.p, count_.p, loc_.p, norm,
+                                                   apart ? field : S);
+    if (apart) {
+        k_apply_stage<<<(T.n + 255) / 256, 256, 0, st>>>(e_.p, T.n, S);
+        FS_LAUNCHED(1);
+    }
     FS_LAUNCHED(wide ? 5 : 4);
 }
 

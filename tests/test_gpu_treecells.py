@@ -102,3 +102,31 @@ def test_nan_reaches_every_target(n, where):
     (x if where == "position" else q)[n // 3] = np.nan
     e = M.E_MQ_Treecode_B200(L, 0.2, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
     assert np.all(np.isnan(e))
+
+
+def test_a_large_sessions_step_is_the_fields_rk4():
+    """1,577,475 points: the stage epilogue runs apart from the field.  One step
+    against RK4 on the host through the same treecode, to rounding."""
+    from multi_species_b200 import decks
+    d = decks.bump_on_tail(h=8)
+    d["remesh_period"] = 100
+    s = M.Simulation(d, "treecode32c")
+    st = s.state()
+    n, dt, L = s.n, d["dt"], d["xmax"]
+    x, p, q = st["xs"], st["ps"], st["q_ws"]
+    qm = np.repeat([sp["q"] / sp["m"] for sp in d["species_list"]], n // 3)
+    f = M.E_MQ_Treecode_B200(L, d["greens_epsilon"], d["mac"], d["degree"], d["max_source"], precision="fp32c")
+    a1 = qm * st["es"]
+    p2 = p + 0.5 * dt * a1
+    x2 = x + 0.5 * dt * p
+    a2 = qm * f.evaluate(x2, x2, q)
+    p3 = p + 0.5 * dt * a2
+    x3 = x + 0.5 * dt * p2
+    a3 = qm * f.evaluate(x3, x3, q)
+    p4 = p + dt * a3
+    x4 = x + dt * p3
+    a4 = qm * f.evaluate(x4, x4, q)
+    s.step(1)
+    out = s.state()
+    assert _rel(out["xs"], x + dt / 6 * (p + 2 * p2 + 2 * p3 + p4)) < 1e-14
+    assert _rel(out["ps"], p + dt / 6 * (a1 + 2 * a2 + 2 * a3 + a4)) < 1e-14
