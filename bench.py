@@ -118,7 +118,7 @@ class ClockSampler:
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={self.idx}", f"--query-gpu={self.FIELDS}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"],
+                                          "--format=csv,noheader,nounits", "-lms", "20"],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             threading.Thread(target=self._read, daemon=True).start()
         except FileNotFoundError:
@@ -236,6 +236,15 @@ def cpu_baseline(deck, seconds: float, treecode: bool = False):
                       f"({dt:.1f} s)"}
 
 
+def cpu_baseline_or_note(deck, seconds, treecode=False):
+    """cpu_baseline, or why it could not be taken (the reference is compiled only
+    where its sources are)."""
+    try:
+        return cpu_baseline(deck, seconds, treecode)
+    except FileNotFoundError as e:
+        return {"unavailable": str(e)}
+
+
 def run_reference(a, rank, world):
     """--impl reference: the reference's CPU direct sum on the host cores."""
     name, deck = workload_deck(a)
@@ -244,8 +253,11 @@ def run_reference(a, rank, world):
     vals = []
     per = max(1.0, a.cpu_seconds / max(1, a.steps + a.warmup))
     tree = int(deck.get("use_treecode", 0)) > 0
-    for _ in range(a.warmup):
-        cpu_baseline(deck, per, tree)
+    try:
+        for _ in range(a.warmup):
+            cpu_baseline(deck, per, tree)
+    except FileNotFoundError as e:
+        return {"impl": "reference", "unavailable": str(e)}
     for _ in range(a.steps):
         vals.append(cpu_baseline(deck, per, tree))
     v = statistics.median(x["value"] for x in vals)
@@ -267,6 +279,7 @@ def run_reference(a, rank, world):
             "e2e": {"value": v, "unit": "pair-interactions/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
 
 
+TREE_CELLS_BYTES_PER_POINT = 40
 KERNEL_OF_FIELD = {"direct32c": "k_pairs32", "direct64": "k_direct64", "treecode32c": "k_near32",
                    "treecode64": "k_far_near64"}
 
@@ -306,12 +319,24 @@ def roofline(a, kern, kl, kms, kwork, total_ms, sm, peaks, peak_src, band_fracti
                          "frac": t_bound / (kms / 1e3), "band_pairs_per_launch": band / kl,
                          "band_fraction": band / kwork, "fp64_band_peak_gpairs": fp64_band_peak / 1e9,
                          "frac_note": "frac = (far pairs / FP32-pipe peak + band pairs / FP64-pipe peak) / kernel "
-                                      "time; achieved and peak are the direct-equivalent rate against the FP32 "
-                                      "bound alone"})
+                                      "time; achieved and peak are the rate of the pairs summed in the launches "
+                                      "against the FP32 bound alone"})
     if a.field == "direct64":
         # two IEEE divisions + one square root + ~11 FP64 ops per pair, no MUFU shortcut
         roof.update({"bound": "fp64-pipe", "peak": None, "frac": None, "mufu_convention": None,
                      "peak_source": "FP64 pipe (reference arithmetic, bit-exact); not a speed-of-light kernel"})
+    elif kern == "k_tree_cells":
+        # near and far sums through cells: compulsory bytes are the sorted
+        # positions, charges, leaves and slots read once for the moments (16 B)
+        # and once for the evaluation (16 B), and the field (8 B)
+        n = (kwork / kl) ** 0.5 if kl else 0.0
+        gbs = TREE_CELLS_BYTES_PER_POINT * n * kl / (kms / 1e3) / 1e9 if kms > 0 else 0.0
+        roof.update({"bound": "hbm", "unit": "GB/s", "achieved": gbs, "peak": peaks["hbm_gbs"],
+                     "frac": gbs / peaks["hbm_gbs"], "mufu_convention": None, "traffic": None,
+                     "pairs_per_launch": kwork / kl if kl else None,
+                     "peak_source": f"{peak_src} copy bandwidth; {TREE_CELLS_BYTES_PER_POINT} compulsory bytes per "
+                                    "point",
+                     "direct_equivalent_per_s": achieved / 1e9})
     elif a.field.startswith("treecode"):
         # actual near-field pairs (counted on the device while profiling) per
         # near-kernel time, against one MUFU rsqrt per pair
@@ -375,6 +400,8 @@ def run_ours(a, rank, world, local_rank):
     pairs, evals = pairs1 - pairs0, evals1 - evals0
     total_ms = float(np.sum(step_ms))
     kern = KERNEL_OF_FIELD[a.field]
+    if a.field.startswith("treecode") and M.profile_read("k_tree_cells")[0]:
+        kern = "k_tree_cells"
     kl, kms, kwork = M.profile_read(kern)
     rl, rms, _ = M.profile_read("remesh")
     sim.close()
@@ -411,30 +438,33 @@ def run_ours(a, rank, world, local_rank):
         if not a.no_e2e:
             res["e2e"] = e2e_plugin(deck, a.field, n, local_rank, a.steps)
         if not a.no_cpu_baseline:
-            res["cpu_baseline"] = cpu_baseline(deck, a.cpu_seconds, a.field.startswith("treecode"))
+            res["cpu_baseline"] = cpu_baseline_or_note(deck, a.cpu_seconds, a.field.startswith("treecode"))
     return res
 
 
 VALUE_NOTE = {
     "direct32c": "pairs are direct-equivalent: N^2 per full evaluation (and U^2 per reduced-grid evaluation) at the "
-                 "accuracy stated in `accuracy`; far pairs (|d| > 16 eps) are summed as an exact FP64 sign part plus a "
-                 "one-term series of analytic error <= v^2/16 (v = eps^2/(d^2+eps^2)) accumulated in FP32, band pairs "
-                 "(|d| <= 16 eps) in FP64",
+                 "accuracy stated in `accuracy`; stage fields are sums over all pairs through FP64 Chebyshev expansions "
+                 "on cells of epsilon / 1.6 (16 terms, 1e-14 of E); the field a call hands out is summed pair by pair "
+                 "within 60 eps (|d| > 16 eps as an exact FP64 sign part plus a one-term series in FP32, the rest in "
+                 "FP64) and through the cells beyond",
     "direct64": "pairs evaluated one by one with the reference's FP64 arithmetic (bit-identical)",
-    "treecode32c": "pairs are direct-equivalent N^2 per evaluation; the treecode evaluates near-field pairs and "
-                   "far-field cluster terms (kernel_evals_per_s)",
-    "treecode64": "pairs are direct-equivalent N^2 per evaluation; the treecode evaluates near-field pairs and "
-                  "far-field cluster terms (kernel_evals_per_s)",
+    "treecode32c": "pairs are direct-equivalent N^2 per evaluation; the treecode sums near-field pairs and far-field "
+                   "cluster terms (kernel_evals_per_s counts them), from 128 points per epsilon on through FP64 "
+                   "Chebyshev cells",
+    "treecode64": "pairs are direct-equivalent N^2 per evaluation; the treecode sums near-field pairs and far-field "
+                  "cluster terms (kernel_evals_per_s counts them), from 16 points per epsilon on through FP64 "
+                  "Chebyshev cells",
 }
 
 # FP64 pipe: 64 FP64 lanes per clock per SM on B200 (half the FP32 lanes).
 FP64_LANES_PER_CLK_PER_SM = 64
-# FP64 thread instructions per pair of k_direct64 (its two IEEE divisions,
-# square root, round, compares and the term: 17.1 DFMA + 12.0 DMUL + 8.0 DADD
-# + 3.1 others), counted by ncu (sm__sass_thread_inst_executed_op_fp64_pred_on
-# over the launch's pairs) on the two-stream deck at 33,153 points; the count
-# per pair does not depend on the size.
-DIRECT64_FP64_INSTR_PER_PAIR = 40.2
+# FP64 thread instructions per pair of k_direct64 (the correctly rounded
+# divisions and square root by products and residual steps: 9.0 DFMA + 10.0 DMUL
+# + 4.0 DADD + 0.1 others), counted by ncu
+# (sm__sass_thread_inst_executed_op_fp64_pred_on over the launch's pairs) on the
+# two-stream deck at 33,153 points; the count per pair does not depend on the size.
+DIRECT64_FP64_INSTR_PER_PAIR = 23.2
 # FP64 instructions per band pair of k_pairs32: d (DADD), d^2 + eps^2 (DFMA),
 # (q/4) d y (two DMUL), y^2 (DMUL), 3 - r y^2 (DFMA) and the accumulation
 # (DFMA), the Newton step's 1/2 folded into q/4; plus one MUFU op.
@@ -693,7 +723,7 @@ def run_batch(a, rank, world, local_rank):
         res["e2e"] = e2e_plugin(big, "direct32c", decks.deck_points(big), local_rank, a.steps)
         res["e2e"]["note"] = "plugin path on the batch's largest instance"
     if not a.no_cpu_baseline:
-        res["cpu_baseline"] = cpu_baseline(big, a.cpu_seconds, False)
+        res["cpu_baseline"] = cpu_baseline_or_note(big, a.cpu_seconds, False)
     return res
 
 

@@ -3,13 +3,16 @@
 //
 // Same tree, lists and moments as the reference, rebuilt every call like the
 // reference does, but on the GPU:
-//   k_tree_keys/sort   particles_x = fmod(x, L) (:235-247), sorted (CUB radix)
+//   k_tree_keys/sort   particles_x = fmod(x, L) (:235-247), sorted by fixed-point
+//                      keys (CUB radix); k_tree_gather and k_tree_runs put points
+//                      of equal keys right
 //   k_build_tree       one CTA, level-synchronous midpoint bisection over the
 //                      root interval [min - 0.1234, max + 0.001] (:506-632,
 //                      :1032-1050): a node with n >= max_source points splits at
 //                      0.5 (x0 + x1), points with x <= mid go left, children only
 //                      when non-empty.  Member ranges are contiguous in sorted
-//                      order, so a split is one binary search.
+//                      order, so a split is one binary search; k_heap_splits
+//                      makes those of the first levels at once.
 //   k_lists            a warp per leaf: the reference's tests from the root
 //                      down (build_interaction_list :663-702) -- any leaf reached
 //                      is near, a node is far when (r_b + r_p) / R < theta with the
@@ -26,6 +29,8 @@
 //   k_far32 + k_near32 FP32-compensated form: far field in FP64 with a
 //                      reciprocal-square-root kernel evaluation, near field as
 //                      FP32 tiles of the near leaves' sources with Kahan sums.
+// With many points per epsilon near and far sums go through cells instead of the
+// last three kernels (csrc/fs_treecells.cu).
 // The kernel of the reference treecode is sqrt(L^2+4 eps^2)/L times the direct
 // sum's (:949, :1008 vs :150); both forms keep that normalisation.
 #include <cub/cub.cuh>
