@@ -25,7 +25,7 @@
 //                      children's, in a fixed order.  cos(k pi/P) comes from the
 //                      host C library.
 //   k_far_near64       per target: far list then near list (Call_BL :904-961,
-//                      Call_Ds :963-1020), the reference's arithmetic in FP64.
+//                      Call_Ds :963-1020) in FP64.
 //   k_far32 + k_near32 FP32-compensated form: far field in FP64 with a
 //                      reciprocal-square-root kernel evaluation, near field as
 //                      FP32 tiles of the near leaves' sources with Kahan sums.
@@ -38,6 +38,7 @@
 #include <cfloat>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "fs_tree.cuh"
@@ -696,57 +697,67 @@ __global__ void __launch_bounds__(kLeafThreads) k_moments(const TNode* __restric
     }
 }
 
-// One term of the reference sum, FP64, same association and roundings as
+// One term of the reference sum over norm = sqrt(L^2 + 4 eps^2) / L,
 // `w * -1.0 * s * (1 - sqrt(deno / (4*s*s*L*L + 4*eps*eps)))`
-// (src/FieldStructure.cpp:940-950, :1000-1010); skipped pairs add nothing.
-__device__ __forceinline__ double tc_term(double w, double xi, double xj, double L, double deno, double four_eps2,
-                                          bool& skip) {
-    double s = ddiv(dsub(xi, xj), L);
-    s = dsub(s, round(s));
-    skip = fabs(dsub(s, 0.5)) < DBL_MIN || fabs(dadd(s, 0.5)) < DBL_MIN || fabs(s) < DBL_MIN;
-    const double den = dadd(dmul(dmul(dmul(dmul(4.0, s), s), L), L), four_eps2);
-    return dmul(dmul(dmul(w, -1.0), s), dsub(1.0, __dsqrt_rn(ddiv(deno, den))));
+// (src/FieldStructure.cpp:940-950, :1000-1010), as w d (1 / (2 sqrt(d^2 + eps^2)) - c):
+// the reciprocal root by the hardware approximation (2^-20) and one step of third
+// order.  The pairs the reference skips (s = 0, +-1/2) are zeros of this form.
+__device__ __forceinline__ double tree_term(double w, double d, double L, double invL, double e2, double c,
+                                            double acc) {
+    d -= L * rint(d * invL);
+    const double r = fma(d, d, e2);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r));
+    const double e = fma(-r * y, y, 1.0);
+    y = fma(y * e, fma(e, 0.375, 0.5), y);
+    return fma(w, d * fma(0.5, y, -c), acc);
 }
 
-// FP64 per target: far field (Call_BL) then near field (Call_Ds), reference
-// arithmetic and order; result through the stage epilogue at the original index.
-__global__ void k_far_near64(const TNode* __restrict__ nodes, const int* __restrict__ meta,
-                             const int* __restrict__ leaf_of, const int* __restrict__ leaves,
-                             const int* __restrict__ far_list, const int* __restrict__ far_n,
-                             const int* __restrict__ near_list, const int* __restrict__ near_n,
-                             const double* __restrict__ mom, const double* __restrict__ consts,
-                             const double* __restrict__ sx, const double* __restrict__ lam,
-                             const int* __restrict__ sidx, int n, int P, double L, double eps, Stage S) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n || meta[2]) return;
-    const double* cheb = consts;
+// FP64 per target: far field (Call_BL) and near field (Call_Ds); result through the
+// stage epilogue at the original index.  kG lanes share a target's terms and add
+// their sums in a tree: a term is a chain of a dozen FP64 operations, and the trees
+// that come here (below 16 points per epsilon) have too few targets to hide it
+// behind one another.  Of the bump-on-tail box, against a thread per target and the
+// reference's two divisions and root per term (the same lists): 2,000 points 624 ->
+// 85 us per field, 10,000 2900 -> 227, 49,000 2740 -> 458; with eight lanes at any
+// size 109, 274 and 460, and in the reference's operations 178, 600 and 1261.
+// Points below which a target has a whole warp: 20,000 take 281 us so and 309 by
+// eight lanes, 25,000 take 340 by eight lanes.
+constexpr int kFarNearWide = 24000;
+template <int kG>
+__global__ void __launch_bounds__(128) k_far_near64(const TNode* __restrict__ nodes, const int* __restrict__ meta,
+                                                    const int* __restrict__ leaf_of, const int* __restrict__ far_list,
+                                                    const int* __restrict__ far_n, const int* __restrict__ near_list,
+                                                    const int* __restrict__ near_n, const double* __restrict__ mom,
+                                                    const double* __restrict__ consts, const double* __restrict__ sx,
+                                                    const double* __restrict__ lam, const int* __restrict__ sidx, int n,
+                                                    int P, double L, double eps, double norm, double cbg, Stage S) {
+    if (meta[2]) return;
+    const int j0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / kG), g = threadIdx.x % kG;
+    const int j = min(j0, n - 1);  // lanes beyond the last target stay for the shuffles
     const int PP = P + 1;
-    const double deno = dadd(dmul(L, L), dmul(dmul(4.0, eps), eps));
-    const double four_eps2 = dmul(dmul(4.0, eps), eps);
+    const double invL = 1.0 / L, e2 = eps * eps;
     const int l = leaf_of[j];
     const double x = sx[j];
     double far = 0.0;
-    for (int f = 0; f < far_n[l]; ++f) {
+    const int terms = far_n[l] * PP;
+    for (int z = g; z < terms; z += kG) {
+        const int f = z / PP, k = z - f * PP;
         const int fi = far_list[(size_t)l * kFarCap + f];
-        const TNode nd = nodes[fi];
-        const double* m = mom + (size_t)fi * (kMaxDegree + 1);
-        for (int k = 0; k < PP; ++k) {
-            const double t = dadd(nd.x0, dmul(dmul(dadd(cheb[k], 1.0), 0.5), dsub(nd.x1, nd.x0)));
-            bool skip;
-            const double v = tc_term(m[k], x, t, L, deno, four_eps2, skip);
-            if (!skip) far = dadd(far, v);
-        }
+        const double x0 = nodes[fi].x0, x1 = nodes[fi].x1;
+        const double t = dadd(x0, dmul(dmul(dadd(consts[k], 1.0), 0.5), dsub(x1, x0)));
+        far = tree_term(mom[(size_t)fi * (kMaxDegree + 1) + k], x - t, L, invL, e2, cbg, far);
     }
     double near = 0.0;
     for (int q = 0; q < near_n[l]; ++q) {
         const TNode nd = nodes[near_list[(size_t)l * kNearCap + q]];
-        for (int i = nd.m0; i <= nd.m1; ++i) {
-            bool skip;
-            const double v = tc_term(lam[i], x, sx[i], L, deno, four_eps2, skip);
-            if (!skip) near = dadd(near, v);
-        }
+#pragma unroll 4
+        for (int i = nd.m0 + g; i <= nd.m1; i += kG) near = tree_term(lam[i], x - sx[i], L, invL, e2, cbg, near);
     }
-    apply_stage(S, sidx[j], dadd(dadd(0.0, far), near));
+    double e = far + near;
+#pragma unroll
+    for (int o = kG / 2; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (g == 0 && j0 < n) apply_stage(S, sidx[j], norm * e);
 }
 
 // FP32-compensated form, far part: FP64 with the kernel written through one
@@ -1369,9 +1380,14 @@ class Treecode final : public FieldEngine {
             FS_LAUNCHED(7);
         } else if (!fp32_) {
             ProfScope prof("k_far_near64", st, last_pairs);
-            k_far_near64<<<(n + 127) / 128, 128, 0, st>>>(nodes_.p, meta_.p, leaf_of_.p, leaves_.p, far_.p, far_n_.p,
-                                                         near_.p, near_n_.p, mom_.p, consts_.p, sx_.p, lam_.p,
-                                                         sidx, n, P_, L_, eps_, stage);
+            auto go = [&](auto lanes) {
+                constexpr int kG = decltype(lanes)::value;
+                k_far_near64<kG><<<(int)(((long long)n * kG + 127) / 128), 128, 0, st>>>(
+                    nodes_.p, meta_.p, leaf_of_.p, far_.p, far_n_.p, near_.p, near_n_.p, mom_.p, consts_.p, sx_.p,
+                    lam_.p, sidx, n, P_, L_, eps_, norm_, cbg_, stage);
+            };
+            if (n < kFarNearWide) go(std::integral_constant<int, 32>{});
+            else go(std::integral_constant<int, 8>{});
             FS_LAUNCHED(8);
         } else {
             {

@@ -130,3 +130,18 @@ def test_a_large_sessions_step_is_the_fields_rk4():
     out = s.state()
     assert _rel(out["xs"], x + dt / 6 * (p + 2 * p2 + 2 * p3 + p4)) < 1e-14
     assert _rel(out["ps"], p + dt / 6 * (a1 + 2 * a2 + 2 * a3 + a4)) < 1e-14
+
+
+@pytest.mark.parametrize("n", [1, 5, 129, 2001, 23_999, 24_000, 24_003])
+def test_fp64_pair_by_pair(n):
+    """Below 16 points per epsilon: targets shared by a warp or by eight lanes, to
+    rounding (as above)."""
+    rng = np.random.default_rng(n)
+    L = 20 * np.pi
+    x = rng.uniform(-L, L, n)
+    m = min(n // 8, 900)                        # fewer coincident points than a leaf holds
+    x[:m] = x[0]
+    x[m: 2 * m] = np.mod(x[0], L) - L / 2       # half a period apart
+    q = rng.normal(size=n) / n
+    e = M.E_MQ_Treecode_B200(L, 0.02, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
+    assert np.max(np.abs(e - O.treecode(L, 0.02, 0.7, 8, 2000, x, q))) < 2e-12 * np.sum(np.abs(q))
