@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(128) k_far_near64(const TNode* __restrict__ no
     const int j0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / kG), g = threadIdx.x % kG;
     const int j = min(j0, n - 1);  // lanes beyond the last target stay for the shuffles
     const int PP = P + 1;
-    const double invL = 1.0 / L, e2 = eps * eps;
+    const double invL = 1.0 / L, e2 = fmax(eps * eps, DBL_MIN);  // a normal root at d = 0, however small eps
     const int l = leaf_of[j];
     const double x = sx[j];
     double far = 0.0;

@@ -145,3 +145,11 @@ def test_fp64_pair_by_pair(n):
     q = rng.normal(size=n) / n
     e = M.E_MQ_Treecode_B200(L, 0.02, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
     assert np.max(np.abs(e - O.treecode(L, 0.02, 0.7, 8, 2000, x, q))) < 2e-12 * np.sum(np.abs(q))
+
+
+def test_fp64_pair_by_pair_with_a_vanishing_epsilon():
+    """epsilon^2 underflows: a point's own pair still adds nothing."""
+    x = np.linspace(0.0, 1.0, 300, endpoint=False)
+    q = np.full(300, -1.0 / 300)
+    e = M.E_MQ_Treecode_B200(1.0, 1e-200, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
+    assert np.max(np.abs(e - O.treecode(1.0, 1e-200, 0.7, 8, 2000, x, q))) < 2e-12
