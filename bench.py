@@ -123,13 +123,22 @@ class ClockSampler:
             threading.Thread(target=self._read, daemon=True).start()
         except FileNotFoundError:
             self.proc = None
+        # the timed region may be shorter than the sampler's start
+        self._await(1, 5.0)
+        self.lines.clear()
         return self
+
+    def _await(self, n, seconds):
+        end = time.perf_counter() + seconds
+        while self.proc and self.proc.poll() is None and len(self.lines) < n and time.perf_counter() < end:
+            time.sleep(0.002)
 
     def _read(self):
         for line in self.proc.stdout:
             self.lines.append(line.strip())
 
     def __exit__(self, *exc):
+        self._await(1, 1.0)
         if self.proc:
             self.proc.terminate()
             try:
