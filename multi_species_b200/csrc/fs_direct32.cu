@@ -1213,16 +1213,6 @@ class Direct32c final : public FieldEngine {
     Direct32c(double L, double eps) : L_(L), eps_(eps) {
         cbg_ = 1 / std::sqrt(L * L + 4 * eps * eps);
         cells_ = cell_plan(L, eps, &plan_);
-        if (cells_) {
-            // the tables depend on L and eps alone; they are there before any
-            // (non-blocking) stream evaluates, captured or not
-            const size_t tab = (size_t)cell_table_offsets(plan_.Mc) * kCellTerms * kCellTerms;
-            tab_.ensure(tab + (size_t)kCellGroup * kCellTerms * kCellTerms);
-            buf_.tab = tab_.p;
-            buf_.child = tab_.p + tab;
-            cell_table(plan_, buf_.tab, buf_.child, nullptr);
-            FS_CUDA(cudaStreamSynchronize(nullptr));
-        }
         // tuning knob: targets per thread of the pair kernel (2, 4 or 8)
         if (const char* v = std::getenv("FS_B200_PAIR_TARGETS")) {
             const int r = std::atoi(v);
@@ -1350,6 +1340,19 @@ class Direct32c final : public FieldEngine {
 
     int* error_flag() override { return err_.p; }
 
+    // The tables depend on L and eps alone; they are there before any
+    // (non-blocking) stream evaluates.  Not made for a batch's members, whose sums
+    // never need them: the wait would be for a launch of the running batch.
+    void prepare_cells() override {
+        if (!cells_ || tab_.p) return;
+        const size_t tab = (size_t)cell_table_offsets(plan_.Mc) * kCellTerms * kCellTerms;
+        tab_.ensure(tab + (size_t)kCellGroup * kCellTerms * kCellTerms);
+        buf_.tab = tab_.p;
+        buf_.child = tab_.p + tab;
+        cell_table(plan_, buf_.tab, buf_.child, nullptr);
+        FS_CUDA(cudaStreamSynchronize(nullptr));
+    }
+
     // A self-field whose pairs beyond 60 to 70 epsilon go through cells, the nearer
     // ones pair by pair as always: the far terms fall as eps^2 / d^2 and so does
     // their rounding, 1e-11 of E for all that lies beyond the window (measured
@@ -1464,6 +1467,7 @@ class Direct32c final : public FieldEngine {
 
     void reserve_cells(int ns) {
         reserve_common();
+        prepare_cells();
         const int M = plan_.M, Mc = plan_.Mc;
         ckeys_.ensure(2 * (size_t)ns);
         iin_.ensure(ns);

@@ -1384,7 +1384,9 @@ struct Sim {
     // the points uses one form throughout).
     void choose_form() {
         via_cells = cells_wanted && field->through_cells(N);
-        if (via_cells) ek.ensure(N);
+        if (!via_cells) return;
+        ek.ensure(N);
+        field->prepare_cells();
     }
 
     // direct-equivalent pairs always; kernel-level evaluations when profiling
