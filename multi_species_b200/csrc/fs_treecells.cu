@@ -35,9 +35,15 @@ constexpr int kP = kCellTerms;
 constexpr int kPP = kP * kP;
 constexpr int kSlotT = 1024;
 
-// Cell of a position of (-L, L) counted without the period: negative left of 0.
+// A position of (-L, L) wrapped into [0, L], from the left of 0 into (0, L]: where
+// x / L underflows to -0, cell_wrap would give 0, a period away from x's neighbours.
+__device__ __forceinline__ double open_wrap(double x, const CellPlan& P) {
+    const double w = cell_wrap(x, P.L);
+    return x < 0.0 && w == 0.0 ? P.L : w;
+}
+// Its cell counted without the period: negative left of 0, rising with x.
 __device__ __forceinline__ int open_cell(double x, const CellPlan& P) {
-    const int c = cell_of(cell_wrap(x, P.L), P);
+    const int c = cell_of(open_wrap(x, P), P);
     return x < 0.0 ? c - P.M : c;
 }
 
@@ -156,7 +162,7 @@ __global__ void __launch_bounds__(256) k_slot_moments(CellPlan P, TreeView T, co
 #pragma unroll
     for (int k = 0; k < kP; ++k) acc[k] = 0.0;
     for (int j = j0 + lane; j < j1; j += 32) {
-        const double xi = fma(cell_wrap(T.sx[j], P.L), P.two_inv_h, -(double)(2 * c + 1));
+        const double xi = fma(open_wrap(T.sx[j], P), P.two_inv_h, -(double)(2 * c + 1));
         double a = T.lam[j], b = a * xi;
         const double x2 = xi + xi;
         acc[0] += a;
@@ -424,7 +430,7 @@ __global__ void __launch_bounds__(256) k_slot_eval(CellPlan P, TreeView T, const
     const int oc = open_cell(x, P);
     const int slot = leaf_slot[l] + min(max(oc - leaf_c0[l], 0), leaf_slot[l + 1] - leaf_slot[l] - 1);
     const int c = oc < 0 ? oc + P.M : oc;
-    const double xi = fma(cell_wrap(x, P.L), P.two_inv_h, -(double)(2 * c + 1));
+    const double xi = fma(open_wrap(x, P), P.two_inv_h, -(double)(2 * c + 1));
     const double E = norm * cheb_sum(loc + (size_t)slot * kP, xi);
     apply_stage(S, T.sidx[j], count[3] ? nan("") : E);
 }

@@ -153,3 +153,24 @@ def test_fp64_pair_by_pair_with_a_vanishing_epsilon():
     q = np.full(300, -1.0 / 300)
     e = M.E_MQ_Treecode_B200(1.0, 1e-200, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
     assert np.max(np.abs(e - O.treecode(1.0, 1e-200, 0.7, 8, 2000, x, q))) < 2e-12
+
+
+@pytest.mark.parametrize("where", ["inside", "last", "first"])
+def test_subnormal_positions_left_of_0(where):
+    """x / L underflows to -0 there: a leaf's cells still rise with x, and such a
+    point has its neighbours' cell.  Bound as above."""
+    rng = np.random.default_rng(7)
+    L, n = 4 * np.pi, 12000
+    tiny = -5e-324 * np.arange(1, 6)
+    if where == "inside":
+        rest = rng.uniform(-0.9 * L, 0.9 * L, n)
+    elif where == "last":       # the tree's last points
+        rest = rng.uniform(-0.9 * L, -1e-3, n)
+    else:                       # a leaf begins with them
+        rest = np.r_[rng.uniform(-0.9 * L, -0.4 * L, n // 2), rng.uniform(0.3 * L, 0.9 * L, n - n // 2)]
+    x = np.r_[rest, tiny]
+    q = rng.normal(size=len(x)) / n
+    q[n:] = 1.0
+    e = M.E_MQ_Treecode_B200(L, L / 700, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
+    ref = O.treecode(L, L / 700, 0.7, 8, 2000, x, q)
+    assert np.max(np.abs(e - ref)) < 2e-12 * np.sum(np.abs(q))
