@@ -724,6 +724,7 @@ __device__ __forceinline__ double tree_term(double w, double d, double L, double
 // Points below which a target has a whole warp: 20,000 take 281 us so and 309 by
 // eight lanes, 25,000 take 340 by eight lanes.
 constexpr int kFarNearWide = 24000;
+constexpr double kCellBox = 640.0;  // L / epsilon from which FP64 sums go through cells (Treecode::through_cells)
 template <int kG>
 __global__ void __launch_bounds__(128) k_far_near64(const TNode* __restrict__ nodes, const int* __restrict__ meta,
                                                     const int* __restrict__ leaf_of, const int* __restrict__ far_list,
@@ -1419,15 +1420,21 @@ class Treecode final : public FieldEngine {
     }
 
    private:
+    const double* halves() const { return consts_.p + 2 * (kMaxDegree + 1); }
     // Sums through cells (csrc/fs_treecells.cu) where leaves hold many points
     // per cell.  The FP32c form changes over where its FP32 near sums are
     // themselves within 6e-10 of the FP64 treecode (1.7e-9 at 32 points per
     // epsilon, 5e-10 at 126, 4e-11 at 2000), so that E does not step there.
-    const double* halves() const { return consts_.p + 2 * (kMaxDegree + 1); }
+    // The FP64 form sums short boxes pair by pair: a cell that the half period
+    // cuts sees the kernel's jump there (48 eps^2 / L^4 in the second derivative),
+    // which leaves up to 4.7e-3 (eps / L)^4 of the charge half a period away.
+    // Error of E, relative L2 against sums in long double, pair by pair and
+    // through cells: 3e-14 and 1.1e-12 at L = 251 epsilon, 3e-14 and 9e-14 at
+    // 400, 1e-13 and 5e-14 at 640, 1.5e-13 and 5e-14 at 1571.
     bool through_cells(int n) const {
         if (!cells_.ready()) return false;
         const double per_eps = n * eps_ / L_;  // points per epsilon at uniform density
-        return fp32_ ? per_eps >= 128 : per_eps >= 16;
+        return fp32_ ? per_eps >= 128 : per_eps >= 16 && L_ >= kCellBox * eps_;
     }
 
     void reserve(int n, int cap_nodes, int cap_leaves) {

@@ -174,3 +174,19 @@ def test_subnormal_positions_left_of_0(where):
     e = M.E_MQ_Treecode_B200(L, L / 700, 0.7, 8, 2000, precision="fp64").evaluate(x, x, q)
     ref = O.treecode(L, L / 700, 0.7, 8, 2000, x, q)
     assert np.max(np.abs(e - ref)) < 2e-12 * np.sum(np.abs(q))
+
+
+@pytest.mark.parametrize("ratio", [33.0, 64.0, 100.0, 251.3, 500.0, 639.0, 641.0])
+@pytest.mark.parametrize("parts", [8, 3, 0])
+def test_fp64_charges_half_a_period_apart(ratio, parts):
+    """All charge in two places half a period apart, where the kernel's second
+    derivative jumps, with several leaves and with one.  Bound: n additions of
+    terms of at most |q| / 2 on either side."""
+    L, n = 4 * np.pi, int(20 * ratio)
+    rng = np.random.default_rng(n + parts)
+    x = 0.1 * L + rng.uniform(0, L / 512, n) + 0.5 * L * (np.arange(n) % 2)
+    q = -rng.uniform(0.5, 1.5, n) * L / n
+    leaf = n // parts if parts else 2 * n
+    e = M.E_MQ_Treecode_B200(L, L / ratio, 0.7, 8, leaf, precision="fp64").evaluate(x, x, q)
+    ref = O.treecode(L, L / ratio, 0.7, 8, leaf, x, q)
+    assert np.max(np.abs(e - ref)) <= n * 2.0 ** -53 * np.sum(np.abs(q))
