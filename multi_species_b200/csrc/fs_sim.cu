@@ -1434,6 +1434,14 @@ struct Sim {
         if (via_cells) FS_CUDA(cudaMemcpyAsync(ek.p, e.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     }
 
+    // Before a remesh, which may fail and then leaves the fields as they are: e is
+    // the field that the points' last stage ended with, not the call's before.
+    void settle_field() {
+        if (!e_stale) return;
+        FS_CUDA(cudaMemcpyAsync(e.p, ek.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
+        e_stale = false;
+    }
+
     // Reduced grid (evaluate_field_uniform_grid): column sums, one field call
     // on the unique x, scatter back to the points.
     void reduced_pre() {
@@ -1495,6 +1503,7 @@ struct Sim {
     }
 
     void remesh_kernels() {
+        settle_field();
         bool any_adaptive = false;
         long long launches = 0;
         for (auto& s : sp) {

@@ -85,3 +85,25 @@ def test_remesh_walk_limit_then_recovers():
     ref.step(2)
     for k in ("xs", "ps", "fs", "q_ws", "es"):
         assert np.array_equal(g.state()[k], ref.state()[k]), k
+
+
+def test_failed_remesh_leaves_the_last_steps_field():
+    """The same in an FP32c session whose stage fields go through cells, the failing
+    step the last of five in one call: E is the fourth step's, to the FP32c sum's
+    error, and the next step starts from it."""
+    d = decks.two_stream(h=6, ph=1, steps=10, remesh_period=5)
+    g, ref = M.Simulation(d, "direct32c"), M.Simulation(d, "direct64")
+    before = M.Simulation(d, "direct64")
+    before.step(4)
+    M.debug_set_wait_limits(0, walk_panels=1)
+    for s in (g, ref):
+        with pytest.raises(M.FsError) as e:
+            s.step(5)
+        assert e.value.code == FS_ERR_WALK
+    M.debug_set_wait_limits(0)
+    assert np.array_equal(ref.state()["es"], before.state()["es"])
+    assert rel(g.state()["es"], ref.state()["es"]) < 1e-8
+    g.step(1)
+    ref.step(1)
+    for k in ("xs", "ps"):
+        assert rel(g.state()[k], ref.state()[k]) < 1e-8, k
