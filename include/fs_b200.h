@@ -196,7 +196,9 @@ fs_status fs_sim_num_points(const fs_sim* sim, int species, int* n);
  * pointer may be NULL (AMRSimulation::scatter / write_to_file). */
 fs_status fs_sim_export(fs_sim* sim, double* xs, double* ps, double* fs, double* q_ws, double* es);
 /* Overwrite positions/velocities of the current state from host arrays (for
- * tests that inject a given state; weights and f are kept). */
+ * tests that inject a given state; weights and f are kept).  es is the field of
+ * the next step's first stage; an exported state imported again goes on bit for
+ * bit as the session that it came from. */
 fs_status fs_sim_import_xp(fs_sim* sim, const double* xs, const double* ps, const double* es);
 fs_status fs_sim_iter(const fs_sim* sim, int* iter, double* t);
 /* Pair interactions evaluated so far (full + reduced), for throughput metrics. */

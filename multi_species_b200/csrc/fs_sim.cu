@@ -797,6 +797,16 @@ __global__ void k_scatter_reduced(int n, const int* __restrict__ inv, const doub
     e[k] = re[inv[k]];
 }
 
+// *differs = 1 where a and b are not the same bits.
+__global__ void k_differs(int n, const double* __restrict__ a, const double* __restrict__ b, int* __restrict__ differs) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n && __double_as_longlong(a[k]) != __double_as_longlong(b[k])) atomicOr(differs, 1);
+}
+__global__ void k_copy_if(int n, const int* __restrict__ flag, const double* __restrict__ a, double* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n && *flag) out[k] = a[k];
+}
+
 // Host-to-device copy that has landed when it returns.  cudaMemcpy from pageable
 // memory may return once the data is staged, with the DMA still queued on the
 // legacy default stream, which the library's non-blocking streams do not wait
@@ -1075,9 +1085,11 @@ struct Sim {
     // step: on lattices of points the FP32 sums' rounding is coherent (1e-9 of E
     // and more, where cells leave 1e-14), and e keeps following the pairwise
     // session to 1e-10, as do positions and velocities, which integrate E.
-    // e_stale: the points have moved since e was formed.
+    // e_stale: the points have moved since e was formed; e_given: e came from the
+    // caller and ek is still to follow (take_given).
     DevBuf<double> ek;
-    bool cells_wanted = true, via_cells = false, e_stale = false;
+    DevBuf<int> e_differs;
+    bool cells_wanted = true, via_cells = false, e_stale = false, e_given = false;
     DevBuf<int> status;
     std::unique_ptr<FieldEngine> field;
     cudaStream_t st = nullptr;
@@ -1428,7 +1440,26 @@ struct Sim {
         if (profiling_enabled()) (void)field->actual_work(st);
         e_stale = false;
     }
-    // e was set from outside the steps: it is the next step's first field too.
+    // e was imported.  Where it is the field that the session would hand out for
+    // these points, bit for bit, the session goes on as the one that handed it out:
+    // its stage field comes through cells again.  Any other e is itself the next
+    // step's first field.  xkB is free between steps.
+    void take_given() {
+        e_given = false;
+        Stage S = base;
+        S.kind = STAGE_STORE;
+        S.out = xkB.p;
+        FieldCall fc = with_drive(FieldCall{x.p, N, qw.p, S, true}, t);
+        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, PairForm::pairwise);
+        fc.stage.out = ek.p;
+        field->eval(fc.x, fc.n, fc.x, fc.q, fc.n, fc.stage, st, PairForm::any);
+        e_differs.ensure(1);
+        FS_CUDA(cudaMemsetAsync(e_differs.p, 0, sizeof(int), st));
+        k_differs<<<blocks(N), kT, 0, st>>>(N, e.p, xkB.p, e_differs.p);
+        k_copy_if<<<blocks(N), kT, 0, st>>>(N, e_differs.p, e.p, ek.p);
+        FS_LAUNCHED(2);
+    }
+    // e was formed from the reduced grid: it is the next step's first field too.
     void first_stage_field() {
         e_stale = false;
         if (via_cells) FS_CUDA(cudaMemcpyAsync(ek.p, e.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
@@ -1752,6 +1783,7 @@ struct Sim {
         remeshing = false;
         reduced_field();
         check_status();
+        e_given = false;
     }
 
     // A step (AMRSimulation::step, AMRSimulation_step.cpp:5-99) is four field
@@ -1767,6 +1799,7 @@ struct Sim {
 
     void pre_call(int c) {
         if (c == 0) {
+            if (e_given && via_cells) take_given();
             Stage S1 = base;
             k_rk_stage1<<<blocks(N), kT, 0, st>>>(N, S1, via_cells ? ek.p : e.p, xkA.p);
             FS_LAUNCHED(1);
@@ -1920,6 +1953,7 @@ fs_status fs_sim_remesh(fs_sim* sim) {
             sim->impl.out->enqueue(sim->impl.st, sim->impl.iter, false, true, sim->impl.N, sim->impl.U, {}, nullptr,
                                    nullptr, nullptr, sim->impl.rx.p, sim->impl.re.p);
         sim->impl.check_status();
+        sim->impl.e_given = false;  // the remesh has formed e
     });
 }
 
@@ -1985,7 +2019,10 @@ fs_status fs_sim_import_xp(fs_sim* sim, const double* xs, const double* ps, cons
         if (ps) v.push_back({S.p.p, ps, b});
         if (es) v.push_back({S.e.p, es, b});
         S.stage_mem.to_device(v, S.st);
-        if (es) S.first_stage_field();
+        if (es) {
+            S.e_stale = false;
+            S.e_given = S.via_cells;
+        }
         FS_CUDA(cudaStreamSynchronize(S.st));
     });
 }

@@ -106,3 +106,41 @@ def test_exported_field_of_a_large_session(ratio, kind):
     t = np.argsort(np.mod(st["xs"], L))[np.unique(np.r_[0, n - 1, rng.integers(0, n, 300)])]
     ref = O.direct_sum(L, L / ratio, st["xs"][t], st["xs"], st["q_ws"])
     assert np.max(np.abs(st["es"][t] - ref)) <= 2e-9 * np.sum(np.abs(st["q_ws"]))
+
+
+@pytest.mark.parametrize("h,ph,backend", [(6, 1, "direct32c"), (7, 0, "direct32c"), (3, 1, "direct32c"),
+                                          (5, 0, "direct64"), (6, 1, "treecode32c"), (7, 1, "treecode32c")])
+def test_an_exported_state_goes_on_bit_for_bit(h, ph, backend):
+    """Positions, velocities and field of a session imported into a fresh one, and
+    into itself, continue as the undisturbed session does."""
+    deck = decks.bump_on_tail if backend.startswith("tree") else decks.two_stream
+    d = deck(h=h, ph=ph)
+    d["remesh_period"] = 100
+    a, b, c = (M.Simulation(d, backend) for _ in range(3))
+    for s in (a, b):
+        s.step(3)
+    st = b.state()
+    for s in (b, c):
+        s.import_xp(st["xs"], st["ps"], st["es"])
+    for _ in range(2):
+        for s in (a, b, c):
+            s.step(2)
+        sa = a.state()
+        for s in (b, c):
+            got = s.state()
+            for k in ("xs", "ps", "es"):
+                assert np.array_equal(got[k], sa[k]), k
+
+
+def test_a_remeshed_state_imported_goes_on_bit_for_bit():
+    d = decks.two_stream(h=6, ph=1, remesh_period=3)
+    a, b = M.Simulation(d, "direct32c"), M.Simulation(d, "direct32c")
+    for s in (a, b):
+        s.step(3)
+    st = b.state()
+    b.import_xp(st["xs"], st["ps"], st["es"])
+    for s in (a, b):
+        s.step(4)
+    sa, sb = a.state(), b.state()
+    for k in ("xs", "ps", "fs", "q_ws", "es"):
+        assert np.array_equal(sa[k], sb[k]), k
