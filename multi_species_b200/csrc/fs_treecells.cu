@@ -439,10 +439,10 @@ __global__ void __launch_bounds__(256) k_slot_eval(CellPlan P, TreeView T, const
 // The stage epilogue of fields formed in another order: a point's stage arrays are
 // six to eight scattered sectors from k_slot_eval, which at 6.3 million points (twice
 // the L2) takes 314 us on average over a step's stages (482 the last); E alone
-// scattered 75 and this 62 to 88.
-__global__ void __launch_bounds__(256) k_apply_stage(const double* __restrict__ E, int n, Stage S) {
+// scattered 75 and this 62 to 88.  Without a tree there is no E, and the state stays.
+__global__ void __launch_bounds__(256) k_apply_stage(TreeView T, const double* __restrict__ E, Stage S) {
     const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < n) apply_stage(S, i, E[i]);
+    if (i < T.n && !T.meta[2]) apply_stage(S, i, E[i]);
 }
 constexpr int kApart = 1 << 20;  // points from which the stage arrays leave the L2
 
@@ -508,7 +508,7 @@ void TreeCells::eval(const TreeView& T, int max_source, double norm, const Stage
     k_slot_eval<<<(T.n + 255) / 256, 256, 0, st>>>(plan_, T, leaf_c0_.p, leaf_slot_.p, count_.p, loc_.p, norm,
                                                    apart ? field : S);
     if (apart) {
-        k_apply_stage<<<(T.n + 255) / 256, 256, 0, st>>>(e_.p, T.n, S);
+        k_apply_stage<<<(T.n + 255) / 256, 256, 0, st>>>(T, e_.p, S);
         FS_LAUNCHED(1);
     }
     FS_LAUNCHED(wide ? 5 : 4);

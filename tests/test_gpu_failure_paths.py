@@ -14,6 +14,7 @@ from multi_species_b200 import decks
 pytestmark = pytest.mark.gpu
 
 FS_ERR_WALK, FS_ERR_TIMEOUT = 4, 6
+FS_ERR_TREE = 9
 
 
 @pytest.fixture(autouse=True)
@@ -107,3 +108,24 @@ def test_failed_remesh_leaves_the_last_steps_field():
     ref.step(1)
     for k in ("xs", "ps"):
         assert rel(g.state()[k], ref.state()[k]) < 1e-8, k
+
+
+@pytest.mark.parametrize("h", [6, 8])
+def test_a_step_without_a_tree_leaves_the_points(h):
+    """More coincident points than a leaf may hold: the tree cannot be split, the
+    step fails and the positions and velocities stay as they were (at h = 8,
+    1,577,475 points, the stage epilogue is a launch of its own)."""
+    d = decks.bump_on_tail(h=h)
+    g = M.Simulation(d, "treecode32c")
+    st = g.state()
+    x, p = st["xs"].copy(), st["ps"].copy()
+    x[:5000], p[:5000] = 1.0, 0.0       # coincident at the second stage
+    g.import_xp(xs=x, ps=p)
+    with pytest.raises(M.FsError) as e:
+        g.step(1)
+    assert e.value.code == FS_ERR_TREE
+    after = g.state()
+    assert np.array_equal(after["xs"], x) and np.array_equal(after["ps"], p)
+    g.import_xp(xs=st["xs"], ps=st["ps"])
+    g.step(1)
+    assert np.all(np.isfinite(g.state()["xs"]))
