@@ -148,18 +148,25 @@ class Hold {
     }
     ~Hold() { end(); }
     char* half(int k) const { return p_.half[k]; }
-    void record(int k, cudaStream_t st) {
-        FS_CUDA(cudaEventRecord(ev_[k], st));
+    // Copies of half k follow on `st`, until its record().
+    void begin(int k, cudaStream_t st) {
+        st_ = st;
+        open_[k] = true;
+    }
+    void record(int k) {
+        FS_CUDA(cudaEventRecord(ev_[k], st_));
         busy_[k] = true;
+        open_[k] = false;
     }
     void wait(int k) {
         if (!busy_[k]) return;
-        busy_[k] = false;
         FS_CUDA(cudaEventSynchronize(ev_[k]));
+        busy_[k] = false;
     }
 
    private:
     void end() {
+        if (open_[0] || open_[1]) (void)cudaStreamSynchronize(st_);  // copies that no event follows
         for (int k = 0; k < 2; ++k) {
             if (busy_[k]) (void)cudaEventSynchronize(ev_[k]);
             if (ev_[k]) cudaEventDestroy(ev_[k]);
@@ -177,7 +184,8 @@ class Hold {
     }
     Piece p_;
     cudaEvent_t ev_[2] = {nullptr, nullptr};
-    bool busy_[2] = {false, false};
+    cudaStream_t st_ = nullptr;
+    bool busy_[2] = {false, false}, open_[2] = {false, false};
 };
 
 // The copies cut into pieces and gathered into loads of at most one half.
@@ -232,9 +240,10 @@ void HostStage::to_host(const std::vector<HostCopy>& copies, cudaStream_t st) {
     }
     Hold h;
     auto issue = [&](size_t k) {
+        h.begin(k & 1, st);
         for (const Chunk& c : v[k])
             FS_CUDA(cudaMemcpyAsync(h.half(k & 1) + c.at, c.src, c.bytes, cudaMemcpyDeviceToHost, st));
-        h.record(k & 1, st);
+        h.record(k & 1);
     };
     for (size_t k = 0; k < std::min<size_t>(2, v.size()); ++k) issue(k);
     for (size_t k = 0; k < v.size(); ++k) {
@@ -250,11 +259,12 @@ void HostStage::to_device(const std::vector<HostCopy>& copies, cudaStream_t st) 
     Hold h;
     for (size_t k = 0; k < v.size(); ++k) {
         h.wait(k & 1);
+        h.begin(k & 1, st);
         for (const Chunk& c : v[k]) {
             shared().threads.copy(h.half(k & 1) + c.at, c.src, c.bytes);
             FS_CUDA(cudaMemcpyAsync(c.dst, h.half(k & 1) + c.at, c.bytes, cudaMemcpyHostToDevice, st));
         }
-        h.record(k & 1, st);
+        h.record(k & 1);
     }
 }
 
