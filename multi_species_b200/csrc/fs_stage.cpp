@@ -5,9 +5,9 @@
 // (21 MB of a 525,825-point state: 2.9 ms).  Here the DMA runs from and to two
 // pinned halves in turn while several threads copy the other half: 1.8 ms for that
 // state (what is left is its page faults), 0.4 in place of 1.1 ms for two arrays
-// of it in; halves of 1 to 8 MB and eight threads were no faster.
+// of it in; halves of 1 to 8 MB and eight threads were no faster.  Where the system
+// refuses pinned memory or events, the copies are plain ones.
 #include <condition_variable>
-#include <deque>
 #include <mutex>
 #include <thread>
 
@@ -23,7 +23,8 @@ constexpr int kCopyThreads = 4;             // the caller's among them
 constexpr size_t kShare = size_t(128) << 10;  // least bytes worth a thread
 
 // Threads that copy pieces of memory for whoever asks; they live while a
-// HostStage does.
+// HostStage does.  Fewer threads than asked for (none, where the system refuses
+// them) only make the caller copy more.
 class CopyThreads {
    public:
     ~CopyThreads() { stop(); }
@@ -33,21 +34,24 @@ class CopyThreads {
             std::memcpy(dst, src, bytes);
             return;
         }
-        Wait w;
         const size_t per = (bytes / parts + 4095) & ~size_t(4095);
+        Piece piece[kCopyThreads];
+        int left = 0;
         {
             std::lock_guard<std::mutex> lk(mu_);
-            while ((int)threads_.size() < kCopyThreads - 1) threads_.emplace_back([this] { work(); });
+            start();
             for (size_t k = 1; k < parts && k * per < bytes; ++k) {
-                todo_.push_back({dst + k * per, src + k * per, std::min(per, bytes - k * per), &w});
-                ++w.left;
+                piece[k] = {dst + k * per, src + k * per, std::min(per, bytes - k * per), &left, nullptr};
+                (last_ ? last_->next : first_) = &piece[k];
+                last_ = &piece[k];
+                ++left;
             }
         }
         cv_.notify_all();
         std::memcpy(dst, src, std::min(per, bytes));
         std::unique_lock<std::mutex> lk(mu_);
-        while (w.left > 0) {
-            if (!todo_.empty()) run_one(lk);
+        while (left > 0) {
+            if (first_) run_one(lk);
             else done_.wait(lk);
         }
     }
@@ -63,34 +67,42 @@ class CopyThreads {
     }
 
    private:
-    struct Wait {
-        int left = 0;
-    };
     struct Piece {
         char* dst;
         const char* src;
         size_t bytes;
-        Wait* w;
+        int* left;
+        Piece* next;
     };
+    void start() {
+        while ((int)threads_.size() < kCopyThreads - 1) {
+            try {
+                threads_.emplace_back([this] { work(); });
+            } catch (...) {
+                return;
+            }
+        }
+    }
     void run_one(std::unique_lock<std::mutex>& lk) {
-        const Piece p = todo_.front();
-        todo_.pop_front();
+        const Piece p = *first_;
+        first_ = p.next;
+        if (!first_) last_ = nullptr;
         lk.unlock();
         std::memcpy(p.dst, p.src, p.bytes);
         lk.lock();
-        if (--p.w->left == 0) done_.notify_all();
+        if (--*p.left == 0) done_.notify_all();
     }
     void work() {
         std::unique_lock<std::mutex> lk(mu_);
         for (;;) {
-            cv_.wait(lk, [&] { return stopping_ || !todo_.empty(); });
-            if (todo_.empty()) return;
+            cv_.wait(lk, [&] { return stopping_ || first_; });
+            if (!first_) return;
             run_one(lk);
         }
     }
     std::mutex mu_;
     std::condition_variable cv_, done_;
-    std::deque<Piece> todo_;
+    Piece *first_ = nullptr, *last_ = nullptr;  // pieces that nobody has taken, in their callers' frames
     std::vector<std::thread> threads_;
     bool stopping_ = false;
 };
@@ -112,8 +124,9 @@ Shared& shared() {
     return *s;
 }
 
-// One staging piece for the length of a copy; no DMA uses it any more when it
-// goes back, whatever happened.
+// One staging piece for the length of a copy, or none where the system refuses
+// pinned memory or events.  No DMA uses it any more when it goes back, whatever
+// happened.
 class Hold {
    public:
     Hold() {
@@ -130,23 +143,23 @@ class Hold {
         }
         if (!p_.half[0]) {
             void* m = nullptr;
-            const cudaError_t e = cudaHostAlloc(&m, 2 * kHalf, cudaHostAllocPortable);
-            if (e != cudaSuccess) {
+            if (cudaHostAlloc(&m, 2 * kHalf, cudaHostAllocPortable) == cudaSuccess) {
+                p_.half[0] = static_cast<char*>(m);
+                p_.half[1] = p_.half[0] + kHalf;
+            } else {
                 (void)cudaGetLastError();
-                give_back();
-                fail(FS_ERR_NOMEM, "allocation of pinned staging memory failed");
             }
-            p_.half[0] = static_cast<char*>(m);
-            p_.half[1] = p_.half[0] + kHalf;
         }
+        ok_ = p_.half[0] != nullptr;
         for (auto& e : ev_)
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            if (ok_ && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
                 (void)cudaGetLastError();
-                end();
-                fail(FS_ERR_CUDA, "event for a staged copy");
+                e = nullptr;
+                ok_ = false;
             }
     }
     ~Hold() { end(); }
+    bool ok() const { return ok_; }
     char* half(int k) const { return p_.half[k]; }
     // Copies of half k follow on `st`, until its record().
     void begin(int k, cudaStream_t st) {
@@ -185,7 +198,7 @@ class Hold {
     Piece p_;
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaStream_t st_ = nullptr;
-    bool busy_[2] = {false, false}, open_[2] = {false, false};
+    bool ok_ = false, busy_[2] = {false, false}, open_[2] = {false, false};
 };
 
 // The copies cut into pieces and gathered into loads of at most one half.
@@ -239,6 +252,11 @@ void HostStage::to_host(const std::vector<HostCopy>& copies, cudaStream_t st) {
         return;
     }
     Hold h;
+    if (!h.ok()) {
+        for (const HostCopy& c : copies) FS_CUDA(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st));
+        FS_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
     auto issue = [&](size_t k) {
         h.begin(k & 1, st);
         for (const Chunk& c : v[k])
@@ -257,6 +275,11 @@ void HostStage::to_device(const std::vector<HostCopy>& copies, cudaStream_t st) 
     const std::vector<std::vector<Chunk>> v = loads_of(copies);
     if (v.empty()) return;
     Hold h;
+    if (!h.ok()) {
+        for (const HostCopy& c : copies) FS_CUDA(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, st));
+        FS_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
     for (size_t k = 0; k < v.size(); ++k) {
         h.wait(k & 1);
         h.begin(k & 1, st);

@@ -5,10 +5,12 @@
 #include "../multi_species_b200/csrc/fs_stage.cpp"
 
 #include <dlfcn.h>
+#include <errno.h>
 #include <pthread.h>
 
 #include <cstdio>
 #include <cstdlib>
+#include <deque>
 #include <map>
 
 namespace {
@@ -159,6 +161,18 @@ int main(int argc, char** argv) {
         failing(fail_copy, [&](HostStage& S) { S.to_device(in, kStream); });
         failing(fail_record, [&](HostStage& S) { S.to_host(out, kStream); });
         failing(fail_record, [&](HostStage& S) { S.to_device(in, kStream); });
+    } else if (what == "refused") {
+        for (bool* b : {&fail_pin, &fail_event, &fail_thread}) {
+            *b = true;
+            {
+                HostStage S;
+                for (size_t n : {size_t(8), 40000 * size_t(8), 3 * kMB, 24 * kMB}) round_trip(S, n, "copy without what is refused");
+            }
+            *b = false;
+            HostStage S;
+            round_trip(S, 24 * kMB, "copy when it is granted again");
+        }
+        expect(pinned.empty(), "staging memory left over");
     } else {
         std::printf("no such scenario\n");
         return 2;
