@@ -75,7 +75,8 @@ void prof_add_work(const char* name, double work);
 // Copies between pageable host arrays and the device through pinned staging
 // memory, the pageable side by several threads (csrc/fs_stage.cpp).  An object
 // that makes such copies holds a HostStage; the staging memory is shared by all of
-// them, at most kStages pieces, and given back when the last one goes.
+// them, at most kStages pieces, comes once their copies are worth it and is given
+// back when the last one goes.
 struct HostCopy {
     void* dst;
     const void* src;
@@ -89,8 +90,8 @@ class HostStage {
     HostStage& operator=(const HostStage&) = delete;
     // Device to host on `st`; the host arrays are filled when it returns.
     void to_host(const std::vector<HostCopy>& copies, cudaStream_t st);
-    // Host to device on `st`; the host arrays have been read when it returns, the
-    // device arrays are written in stream order.
+    // Host to device on `st`, in stream order; the host arrays have been read once
+    // the stream has been waited for.
     void to_device(const std::vector<HostCopy>& copies, cudaStream_t st);
 };
 

@@ -173,6 +173,21 @@ int main(int argc, char** argv) {
             round_trip(S, 24 * kMB, "copy when it is granted again");
         }
         expect(pinned.empty(), "staging memory left over");
+    } else if (what == "short lives") {
+        for (int k = 0; k < 50; ++k) {  // one object after another
+            HostStage S;
+            round_trip(S, 2 * kMB, "copy of a short life");
+        }
+        expect(pins == 0 && threads == 0, "staging memory or threads for objects of one call");
+        HostStage A;
+        for (int k = 0; k < 30; ++k) {
+            HostStage B;
+            round_trip(B, 2 * kMB, "copy beside a long life");
+        }
+        expect(pins == 1, "no staging memory for many calls, or more than one piece");
+        const int at = records;
+        round_trip(A, 2 * kMB, "staged copy");
+        expect(records > at, "a copy past its staging memory");
     } else {
         std::printf("no such scenario\n");
         return 2;

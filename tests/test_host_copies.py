@@ -19,7 +19,7 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["failing copies", "refused"])
+@pytest.mark.parametrize("scenario", ["failing copies", "refused", "short lives"])
 def test_host_copies(harness, scenario):
     r = subprocess.run([harness, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
