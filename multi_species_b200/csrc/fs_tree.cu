@@ -724,7 +724,7 @@ __device__ __forceinline__ double tree_term(double w, double d, double L, double
 // Points below which a target has a whole warp: 20,000 take 281 us so and 309 by
 // eight lanes, 25,000 take 340 by eight lanes.
 constexpr int kFarNearWide = 24000;
-constexpr double kCellBox = 640.0;  // L / epsilon from which FP64 sums go through cells (Treecode::through_cells)
+constexpr double kCellBox = 640.0;  // L / epsilon from which FP64 sums go through cells (Treecode::cells_take)
 template <int kG>
 __global__ void __launch_bounds__(128) k_far_near64(const TNode* __restrict__ nodes, const int* __restrict__ meta,
                                                     const int* __restrict__ leaf_of, const int* __restrict__ far_list,
@@ -1373,7 +1373,7 @@ class Treecode final : public FieldEngine {
             launch_moments<false>(P_ + 1, cap_leaves, st, nodes_.p, meta_.p, leaves_.p, consts_.p, halves(), sx_.p,
                                   lam_.p, arrived_.p, mom_.p);
         k_copy_meta_error<<<1, 1, 0, st>>>(meta_.p, err_.p);
-        if (through_cells(n)) {
+        if (cells_take(n)) {
             const TreeView T{nodes_.p, leaves_.p, meta_.p, leaf_of_.p, far_.p, far_n_.p, near_.p, near_n_.p,
                              mom_.p, consts_.p, sx_.p, lam_.p, sidx, n, P_, cap_leaves};
             ProfScope prof("k_tree_cells", st, last_pairs);
@@ -1431,7 +1431,7 @@ class Treecode final : public FieldEngine {
     // Error of E, relative L2 against sums in long double, pair by pair and
     // through cells: 3e-14 and 1.1e-12 at L = 251 epsilon, 3e-14 and 9e-14 at
     // 400, 1e-13 and 5e-14 at 640, 1.5e-13 and 5e-14 at 1571.
-    bool through_cells(int n) const {
+    bool cells_take(int n) const {
         if (!cells_.ready()) return false;
         const double per_eps = n * eps_ / L_;  // points per epsilon at uniform density
         return fp32_ ? per_eps >= 128 : per_eps >= 16 && L_ >= kCellBox * eps_;

@@ -17,7 +17,7 @@
 //   k_slot_eval     E_j = norm * sum_l A_s[l] T_l(place), stage epilogue
 // Near lists, far lists and cluster moments are the treecode's own; only how
 // their sums are formed differs (E of long boxes changes by 2e-15 against pair by pair
-// in FP64; of boxes below 640 epsilon more: Treecode::through_cells, csrc/fs_tree.cu).
+// in FP64; of boxes below 640 epsilon more: Treecode::cells_take, csrc/fs_tree.cu).
 //
 // Measured per evaluation, near and far pair by pair against this: 395,523 points
 // in FP64 9.8 ms (of 9.97) and 0.12; 6,300,675 points in FP32c 13.4 ms and 0.34

@@ -190,3 +190,18 @@ def test_fp64_charges_half_a_period_apart(ratio, parts):
     e = M.E_MQ_Treecode_B200(L, L / ratio, 0.7, 8, leaf, precision="fp64").evaluate(x, x, q)
     ref = O.treecode(L, L / ratio, 0.7, 8, leaf, x, q)
     assert np.max(np.abs(e - ref)) <= n * 2.0 ** -53 * np.sum(np.abs(q))
+
+
+@pytest.mark.parametrize("h,ph,backend", [(6, 1, "treecode64"), (8, 0, "treecode32c")])
+def test_a_session_sums_each_field_once(h, ph, backend):
+    """Two steps in one call launch what two calls of one step launch."""
+    from multi_species_b200 import decks
+    d = decks.bump_on_tail(h=h, ph=ph)
+    d["remesh_period"] = 100
+    s = M.Simulation(d, backend)
+    s.step(1)
+    n = [M.kernel_launches()]
+    for k in (1, 2):
+        s.step(k)
+        n.append(M.kernel_launches())
+    assert n[2] - n[1] == 2 * (n[1] - n[0])
