@@ -67,7 +67,8 @@ fs_status fs_field_create(const fs_field_params* params, fs_field** out) {
             case FS_FIELD_DIRECT64: f->engine.reset(fsb::make_direct64(P.L, P.epsilon)); break;
             case FS_FIELD_DIRECT32C:
                 f->engine.reset(fsb::make_direct32c(P.L, P.epsilon));
-                f->engine->prepare_cells();
+                f->engine->prepare_cells(f->st);
+                FS_CUDA(cudaStreamSynchronize(f->st));  // callers evaluate on streams of their own
                 break;
             case FS_FIELD_DIRECT64_OPEN: f->engine.reset(fsb::make_direct64_open(P.epsilon)); break;
             case FS_FIELD_TREECODE64:

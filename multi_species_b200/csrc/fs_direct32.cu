@@ -1227,7 +1227,7 @@ class Direct32c final : public FieldEngine {
             last_pairs = (double)nt * (double)ns;
             last_nt_ = 0;
             fin_ = Fin{};
-            reserve_cells(ns);
+            reserve_cells(ns, st);
             cell_field(plan_, buf_, d_t, nt, d_s, d_q, ns, stage, err_.p, st);
             return;
         }
@@ -1340,17 +1340,15 @@ class Direct32c final : public FieldEngine {
 
     int* error_flag() override { return err_.p; }
 
-    // The tables depend on L and eps alone; they are there before any
-    // (non-blocking) stream evaluates.  Not made for a batch's members, whose sums
-    // never need them: the wait would be for a launch of the running batch.
-    void prepare_cells() override {
+    // The tables depend on L and eps alone.  Not made for a batch's members, whose
+    // sums never need them.
+    void prepare_cells(cudaStream_t st) override {
         if (!cells_ || tab_.p) return;
         const size_t tab = (size_t)cell_table_offsets(plan_.Mc) * kCellTerms * kCellTerms;
         tab_.ensure(tab + (size_t)kCellGroup * kCellTerms * kCellTerms);
         buf_.tab = tab_.p;
         buf_.child = tab_.p + tab;
-        cell_table(plan_, buf_.tab, buf_.child, nullptr);
-        FS_CUDA(cudaStreamSynchronize(nullptr));
+        cell_table(plan_, buf_.tab, buf_.child, st);
     }
 
     // A self-field whose pairs beyond 60 to 70 epsilon go through cells, the nearer
@@ -1371,13 +1369,11 @@ class Direct32c final : public FieldEngine {
         PairJob job;
         if (!prepare(d_x, n, d_x, d_q, n, stage, st, tpc, &job)) return;
         // the cells' part, on the sorted sources
-        reserve_cells(n);
+        reserve_cells(n, st);
         const size_t rest = cell_rest_table_size(plan_);
         if (!rest_.p) {
-            // once, before any (non-blocking) stream reads it
             rest_.ensure(rest);
-            cell_rest_table(plan_, buf_.tab, rest_.p, nullptr);
-            FS_CUDA(cudaStreamSynchronize(nullptr));
+            cell_rest_table(plan_, buf_.tab, rest_.p, st);
         }
         locc2_.ensure(2 * (size_t)plan_.Mc * kCellTerms);
         xs_.ensure(n);
@@ -1465,9 +1461,9 @@ class Direct32c final : public FieldEngine {
         bandcount_.ensure(1);
     }
 
-    void reserve_cells(int ns) {
+    void reserve_cells(int ns, cudaStream_t st) {
         reserve_common();
-        prepare_cells();
+        prepare_cells(st);
         const int M = plan_.M, Mc = plan_.Mc;
         ckeys_.ensure(2 * (size_t)ns);
         iin_.ensure(ns);

@@ -299,8 +299,8 @@ class FieldEngine {
     virtual void eval(const double* d_targets, int nt, const double* d_sources, const double* d_q,
                       int ns, const Stage& stage, cudaStream_t st, PairForm form = PairForm::any) = 0;
     // Makes what sums through cells need beforehand, where the engine has such
-    // (ahead of evaluations that may be captured).
-    virtual void prepare_cells() {}
+    // (ahead of evaluations that may be captured), on `st`.
+    virtual void prepare_cells(cudaStream_t st) { (void)st; }
     // Whether an evaluation of n sources in form `any` is summed otherwise than in
     // form `pairwise`, through cells (the treecode sums in one way whatever the form).
     virtual bool through_cells(int n) const {

@@ -1398,7 +1398,7 @@ struct Sim {
         via_cells = cells_wanted && field->through_cells(N);
         if (!via_cells) return;
         ek.ensure(N);
-        field->prepare_cells();
+        field->prepare_cells(st);
     }
 
     // direct-equivalent pairs always; kernel-level evaluations when profiling

@@ -482,13 +482,13 @@ void TreeCells::eval(const TreeView& T, int max_source, double norm, const Stage
     mom_.ensure((size_t)cap_slots * kP);
     loc_.ensure((size_t)cap_slots * kP);
     if (!tab_.p) {
-        // once, before any (non-blocking) stream reads it: it depends on L and
-        // epsilon alone
+        // once: it depends on L and epsilon alone.  On this stream, without a wait:
+        // evaluations of an engine share its buffers and come one after another,
+        // whatever their streams
         tab_.ensure((size_t)plan_.M * kPP + kPP + kP);
-        cell_offset_table(plan_, tab_.p, nullptr);
-        k_node_table<<<1, kPP, 0, nullptr>>>(tab_.p + (size_t)plan_.M * kPP);
+        cell_offset_table(plan_, tab_.p, st);
+        k_node_table<<<1, kPP, 0, st>>>(tab_.p + (size_t)plan_.M * kPP);
         FS_LAUNCHED(1);
-        FS_CUDA(cudaStreamSynchronize(nullptr));
     }
     k_leaf_slots<<<1, kSlotT, 0, st>>>(plan_, T, width, leaf_c0_.p, leaf_slot_.p, leaf_chunk_.p, chunk_leaf_.p,
                                        chunk_c_.p, arrived_.p, count_.p);

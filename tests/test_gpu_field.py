@@ -212,3 +212,40 @@ def test_fp32c_treecode_session_is_deterministic():
         s.close()
     for k in ("xs", "ps", "es"):
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+def test_first_use_waits_for_nobody_elses_work():
+    """A field handle's creation and its first evaluation on the caller's stream
+    return while other work runs on the legacy default stream."""
+    import time
+
+    import torch
+    L, n = 20 * np.pi, 60000
+    x = torch.rand(n, dtype=torch.float64, device="cuda") * L
+    q, es, st = torch.full_like(x, -L / n), torch.zeros_like(x), torch.cuda.Stream()
+    make = (lambda: M.E_MQ_Treecode_B200(L, 0.02, 0.7, 8, 2000, precision="fp64"),
+            lambda: M.E_MQ_DirectSum_B200(L, 0.02, "fp32c"))
+
+    def evaluate(f):
+        f.evaluate_device(es.data_ptr(), x.data_ptr(), n, x.data_ptr(), q.data_ptr(), n, st.cuda_stream)
+    for m in make:          # the kernels are loaded
+        f = m()
+        evaluate(f)
+        torch.cuda.synchronize()
+        f.close()
+    tree = make[0]()        # (its constants are copied on the legacy stream, as ever)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    torch.cuda._sleep(int(6e8))
+    b.record()
+    t = time.perf_counter()
+    evaluate(tree)
+    direct = make[1]()
+    took = time.perf_counter() - t
+    torch.cuda.synchronize()
+    slept = a.elapsed_time(b) * 1e-3
+    assert slept > 0.1 and took < 0.5 * slept, (took, slept)
+    evaluate(direct)
+    torch.cuda.synchronize()
+    direct.close()
+    tree.close()
