@@ -1465,8 +1465,9 @@ struct Sim {
         if (via_cells) FS_CUDA(cudaMemcpyAsync(ek.p, e.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     }
 
-    // Before a remesh, which may fail and then leaves the fields as they are: e is
-    // the field that the points' last stage ended with, not the call's before.
+    // Before a remesh, which may fail and then leaves the fields as they are, and
+    // after a call that failed: e is the field that the points' last stage ended
+    // with, not the call's before.
     void settle_field() {
         if (!e_stale) return;
         FS_CUDA(cudaMemcpyAsync(e.p, ek.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
@@ -2003,7 +2004,7 @@ fs_status fs_sim_export(fs_sim* sim, double* xs, double* ps, double* fs, double*
         if (!sim) fsb::fail(FS_ERR_ARG, "null sim");
         auto& S = sim->impl;
         FS_CUDA(cudaSetDevice(S.prm.device));
-        if (es) S.export_field();  // a step that failed midway through its call
+        if (es) S.settle_field();  // after a call that failed midway
         S.copy_out(S.st, xs, ps, fs, q_ws, es);
     });
 }

@@ -129,3 +129,25 @@ def test_a_step_without_a_tree_leaves_the_points(h):
     g.import_xp(xs=st["xs"], ps=st["ps"])
     g.step(1)
     assert np.all(np.isfinite(g.state()["xs"]))
+
+
+@pytest.mark.parametrize("steps", [1, 3])
+def test_large_session_timeout_is_reported(steps):
+    """A session of 66,049 points: stage fields through cells, the field handed out
+    from windows of pairs.  The failed call is reported, the state can still be
+    read, and given back what it was the session steps as an undisturbed one."""
+    d = decks.two_stream(h=7, ph=0, remesh_period=100)
+    g, ref = M.Simulation(d, "direct32c"), M.Simulation(d, "direct32c")
+    st = g.state()
+    M.debug_set_wait_limits(0, mbar_polls=0)
+    with pytest.raises(M.FsError) as e:
+        g.step(steps)
+    assert e.value.code == FS_ERR_TIMEOUT
+    g.state()
+    M.debug_set_wait_limits(0)
+    g.import_xp(st["xs"], st["ps"], st["es"])
+    g.step(2)
+    ref.step(2)
+    a, b = g.state(), ref.state()
+    for k in ("xs", "ps", "fs", "q_ws", "es"):
+        assert np.array_equal(a[k], b[k]), k
