@@ -131,6 +131,25 @@ def test_a_step_without_a_tree_leaves_the_points(h):
     assert np.all(np.isfinite(g.state()["xs"]))
 
 
+@pytest.mark.parametrize("n", [90_000, 200_000])
+def test_cell_wait_timeout_then_recovers(n):
+    """The bounded waits of the sums between cells (n L / epsilon above 2e7)."""
+    rng = np.random.default_rng(n)
+    L = 4 * np.pi
+    x = rng.uniform(-L, 2 * L, n)
+    q = rng.normal(size=n) / n
+    f = M.E_MQ_DirectSum_B200(L, 0.05, "fp32c")
+    ref = f.evaluate(x, x, q)
+    M.debug_set_wait_limits(0, mbar_polls=0)
+    with pytest.raises(M.FsError) as e:
+        f.evaluate(x, x, q)
+    assert e.value.code == FS_ERR_TIMEOUT
+    M.debug_set_wait_limits(0)
+    for _ in range(2):
+        assert np.array_equal(f.evaluate(x, x, q), ref)
+    f.close()
+
+
 @pytest.mark.parametrize("steps", [1, 3])
 def test_large_session_timeout_is_reported(steps):
     """A session of 66,049 points: stage fields through cells, the field handed out
