@@ -331,9 +331,12 @@ def roofline(a, kern, kl, kms, kwork, total_ms, sm, peaks, peak_src, band_fracti
                                       "time; achieved and peak are the rate of the pairs summed in the launches "
                                       "against the FP32 bound alone"})
     if a.field == "direct64":
-        # two IEEE divisions + one square root + ~11 FP64 ops per pair, no MUFU shortcut
-        roof.update({"bound": "fp64-pipe", "peak": None, "frac": None, "mufu_convention": None,
-                     "peak_source": "FP64 pipe (reference arithmetic, bit-exact); not a speed-of-light kernel"})
+        # the reference's correctly rounded values, its divisions and square root by
+        # products and residual steps
+        peak = sm * FP64_LANES_PER_CLK_PER_SM * clk_hz / DIRECT64_FP64_INSTR_PER_PAIR
+        roof.update({"bound": "fp64-pipe", "peak": peak / 1e9, "frac": achieved / peak, "mufu_convention": None,
+                     "peak_source": f"{sm} SMs x {FP64_LANES_PER_CLK_PER_SM} FP64 lanes/clk x sm_max_mhz {mhz:.0f} / "
+                                    f"{DIRECT64_FP64_INSTR_PER_PAIR} FP64-pipe instructions per pair"})
     elif kern == "k_tree_cells":
         # near and far sums through cells: compulsory bytes are the sorted
         # positions, charges, leaves and slots read once for the moments (16 B)
@@ -462,7 +465,8 @@ VALUE_NOTE = {
                    "cluster terms (kernel_evals_per_s counts them), from 128 points per epsilon on through FP64 "
                    "Chebyshev cells",
     "treecode64": "pairs are direct-equivalent N^2 per evaluation; the treecode sums near-field pairs and far-field "
-                  "cluster terms (kernel_evals_per_s counts them), from 16 points per epsilon on through FP64 "
+                  "cluster terms (kernel_evals_per_s counts them), in boxes of 640 epsilon and more from 16 points "
+                  "per epsilon on through FP64 "
                   "Chebyshev cells",
 }
 

@@ -7,8 +7,9 @@
 // so on cells no wider than eps / 1.6 its dependence on the source's and on
 // the target's place in their cells is a polynomial to FP64 rounding: with
 // half-width a the Chebyshev series converges like rho^-n, rho = eps/a +
-// sqrt((eps/a)^2 + 1) = 6.5, and 16 terms leave 1e-13 (measured 1e-14 to
-// 4e-13 relative L2 in E).  The sum over all pairs becomes
+// sqrt((eps/a)^2 + 1) = 6.5: 16 terms leave 6.5^-16 = 1e-13 of a pair's charge at
+// most, 3e-14 as formed (within a cell; 4e-15 from the second neighbour on).  The
+// sum over all pairs becomes
 //   k_cell_moments / k_cell_gather  M_J[k] = sum_{j in J} q_j T_k(xi_j)
 //   k_cell_pairs                    A_I[l] = sum_J sum_k T^{(I-J)}[k][l] M_J[k]
 //   k_cell_eval                     E_i = sum_l A_I[l] T_l(xi_i)
@@ -20,11 +21,14 @@
 //
 // The pair sums run on two levels.  16 cells form a group; the near groups
 // (-1, 0, +1) and the group half a period away, whose pairs change their
-// periodic image, interact cell by cell, the rest group by group, where the
-// singularity is at least a group width away.  G and G' are continuous at
-// d = +-L/2 and G'' jumps by 48 eps^2 / L^4 there; only the one cell pair per
-// target cell that straddles it sees the jump (below 2e-12 of E at L = 32 eps
-// with the least cell count, 256, and falling as (eps/L)^2 / cells^3).
+// periodic image, interact cell by cell, the rest group by group.  Of those the
+// nearest are a group's width apart, 10 eps: three half-widths from a group's
+// middle to the other's points, rho = 5.8, and 5.8^-16 = 6e-13 of what of a term is
+// not a polynomial (eps^2 / d^2 of it), 5.4e-14 of the charge as formed.  G and G'
+// are continuous at d = +-L/2 and G'' jumps by 48 eps^2 / L^4 there; only the one
+// cell pair per target cell that straddles it sees the jump, which leaves of that
+// cell's charge up to 1.3e-10 at L = 33 eps, where the pairwise FP32 terms round by
+// as much, 8e-13 at 251 and 2e-14 at 640.  Measured relative L2 in E: 1e-14 to 4e-13.
 //
 // T^{(m)} depends on L and eps alone: it is formed once per (L, eps).  Every
 // sum has a fixed association, so results are a function of the inputs.
