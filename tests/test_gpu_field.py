@@ -217,8 +217,6 @@ def test_fp32c_treecode_session_is_deterministic():
 def test_first_use_waits_for_nobody_elses_work():
     """A field handle's creation and its first evaluation on the caller's stream
     return while other work runs on the legacy default stream."""
-    import time
-
     import torch
     L, n = 20 * np.pi, 60000
     x = torch.rand(n, dtype=torch.float64, device="cuda") * L
@@ -233,19 +231,18 @@ def test_first_use_waits_for_nobody_elses_work():
         evaluate(f)
         torch.cuda.synchronize()
         f.close()
-    tree = make[0]()        # (its constants are copied on the legacy stream, as ever)
-    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    a.record()
-    torch.cuda._sleep(int(6e8))
-    b.record()
-    t = time.perf_counter()
-    evaluate(tree)
-    direct = make[1]()
-    took = time.perf_counter() - t
-    torch.cuda.synchronize()
-    slept = a.elapsed_time(b) * 1e-3
-    assert slept > 0.1 and took < 0.5 * slept, (took, slept)
-    evaluate(direct)
-    torch.cuda.synchronize()
-    direct.close()
-    tree.close()
+    returned = []
+    for _ in range(3):      # (an allocation may take long by itself)
+        tree = make[0]()    # (its constants are copied on the legacy stream, as ever)
+        torch.cuda._sleep(int(6e8))
+        done = torch.cuda.Event()
+        done.record()
+        evaluate(tree)
+        direct = make[1]()
+        returned.append(not done.query())
+        torch.cuda.synchronize()
+        evaluate(direct)
+        torch.cuda.synchronize()
+        direct.close()
+        tree.close()
+    assert any(returned)
